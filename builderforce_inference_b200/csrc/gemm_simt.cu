@@ -2,8 +2,9 @@
 // types and every size: C[M,N] = A[M,K] * W[N,K]^T with W stored [out, in] row-major as the
 // reference stores it (crates/bfi-core/src/cpu.rs:78-90, 498-514).
 //
-// These kernels are the whole of the true 32-bit path (no tensor-core mode is involved) and the
-// fallback of the bfloat16 path for shapes and dtype pairs the tensor-core kernels refuse.
+// These kernels are the 32-bit path's products of up to 16 rows (bound by reading W) and of the sizes that
+// gemm_split.cu refuses, and the fallback of the bfloat16 path for shapes and dtype pairs the tensor-core
+// kernels refuse.
 //
 // Epilogues:
 //   0  C = acc                         (C in c_dtype)

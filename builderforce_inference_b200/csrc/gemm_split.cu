@@ -1,0 +1,486 @@
+// float32 matrix product on the fifth-generation tensor cores, without giving up a bit of the operands:
+// C[M,N] = A[M,K] * W[N,K]^T for float32 A and W.
+//
+// A float32 value is the sum of three bfloat16 terms, x = h + m + l, exactly (8 + 8 + 8 significant bits; every
+// term the rounding of what the terms before it leave).  A product of two values is then nine products of
+// terms, of which the six that reach 2^-18 of it are computed, each exact in float32:
+//     h h  (a chain of its own)      h m + m h + m m + h l + l h  (a second one)
+// What is left out (m l, l m, l l) is at most 2^-26 of a product each, with either sign: a quarter of one
+// float32 rounding.  The tensor cores add with truncation, so a long chain of additions would drift; the h h
+// chain is therefore cut every 128 values of k and added, rounded to nearest, to float32 sums in registers
+// (the second chain is 2^-8 of the first, and so is its drift).  Distance from a 64-bit product, relative to
+// the result's 2-norm, beside the sequential float32 multiply-adds of gemm_simt.cu on the same data (normal values;
+// in brackets A's spread over e^3):
+//     K 1000: 1.3e-7 against 5.6e-7 (1.8e-7, 4.2e-7)      K 2560: 1.4e-7 against 9.0e-7 (2.1e-7, 7.4e-7)
+//     K 9728: 1.6e-7 against 1.8e-6 (2.2e-7, 1.4e-6)      K 256: 1.3e-7 against 2.8e-7 (2.6e-7, 2.4e-7: GS_MIN_K)
+// A result that is not finite (an infinite or NaN operand, or one beyond
+// bfloat16's range) is computed again with float32 multiply-adds, so these come out as they always did.
+//
+// One block per tile of 128 tokens x up to 256 features (and per split of K):
+//   warps 0-7  read float32 rows of A and W, 32 values of k at a time and one block of k ahead, split them and
+//              write the three terms into the ring (64-byte swizzled rows); every fourth block they fetch the
+//              h h chain out of tensor memory into their registers, while the second chain's products of the
+//              next block keep the tensor cores busy
+//   warps 8-11 one lane of warp 8 issues the products: 12 tcgen05.mma of M = 128 per block of 32 k
+// With K split, the blocks of a tile form a cluster and add their partial tiles in split order out of each
+// other's shared memory.
+//
+// What bounds it: the tensor pipe (six bfloat16 products for one of float32, 1657 / 6 = 276 TFLOP/s of the
+// measured peak); a block of 32 k takes 1.84 us at 256 features, 12 instructions of 0.12 us and what the workers'
+// shared-memory traffic adds.  The float32 multiply-adds of 148 x 128 lanes are 74 TFLOP/s; gemm_simt.cu reaches 25.
+// Tokens x features x k, gemm_simt.cu -> this kernel:
+//     1134 x 6144 x 2560    1435 -> 269 us (133 TFLOP/s)      1134 x 2560 x 9728    2749 -> 408 us (138 TFLOP/s)
+//      333 x 2560 x 4096     648 ->  69 us                      64 x 19456 x 2560    515 -> 130 us
+//       24 x 6144 x 2560     183 ->  37 us                      40 x 2560 x 2560     181 ->  23 us
+//
+// Every wait on an mbarrier is bounded: one that runs out records BFI_STATUS_TIMEOUT and the block returns.
+#include "tcgen05.cuh"
+
+#define EPI_STORE 0
+#define EPI_ACCUMULATE 1
+#define EPI_SWIGLU 2
+
+#define GS_TOKENS 128
+#define GS_FEATS 256                                  // widest tile, and the distance of the two chains in tensor memory
+#define GS_BK 32                                      // k values per block: 64 bytes of a term
+#define GS_CHAIN 4                                    // blocks of k between two fetches of the h h chain
+#define GS_STAGES 3
+#define GS_MIN_K 512                                  // shorter sums: the multiply-adds' own rounding can be as small as the truncation of a chain
+#define GS_WORKERS 8
+#define GS_THREADS (GS_WORKERS * 32 + 128)             // a worker holds 128 sums: the registers are split 232 / 40 between the warpgroups
+#define GS_A_TERM (GS_TOKENS * GS_BK * 2)
+#define GS_W_TERM (GS_FEATS * GS_BK * 2)
+#define GS_STAGE_BYTES (3 * (GS_A_TERM + GS_W_TERM))  // 72 KB
+#define GS_OUT_LD (GS_FEATS + 4)                      // floats between rows of the tile on its way out
+#define GS_SMEM ((size_t)GS_STAGES * GS_STAGE_BYTES + 1024 + 128)
+static_assert(GS_TOKENS * GS_OUT_LD * 4 <= GS_STAGES * GS_STAGE_BYTES, "the tile leaves through the ring");
+
+// K-major tile with 64-byte rows and the 64-byte swizzle: groups of 8 rows 512 bytes apart, layout type 4.
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
+// Two values into their terms: h, m and l of both, packed.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    h = *reinterpret_cast<uint32_t*>(&t);
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xffff0000u);
+    t = __floats2bfloat162_rn(a, b);
+    m = *reinterpret_cast<uint32_t*>(&t);
+    a -= __uint_as_float(m << 16);
+    b -= __uint_as_float(m & 0xffff0000u);
+    t = __floats2bfloat162_rn(a, b);
+    l = *reinterpret_cast<uint32_t*>(&t);
+}
+
+// One output by float32 multiply-adds, k rising: for results that are not finite.
+__device__ __noinline__ float dot_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
+    float s = 0.0f;
+    for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+    return s;
+}
+
+// All threads of the tile's blocks meet.
+__device__ __forceinline__ void gs_meet(int ksplit) {
+    if (ksplit > 1)
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+        asm volatile("bar.sync 0, %0;" ::"n"(GS_THREADS) : "memory");
+}
+
+__global__ void __launch_bounds__(GS_THREADS, 1)
+gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, void* __restrict__ C, int c_dtype,
+                  long ldc, int M, int N, int K, int tile_n, int kblocks_per_split, int epilogue, int vec_ok, GateAct gate,
+                  int* __restrict__ status) {
+    const uint32_t spin_limit = TC_SPIN_LIMIT;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)GS_STAGES * GS_STAGE_BYTES);
+    uint64_t* empty = full + GS_STAGES;
+    uint64_t* chain_full = empty + GS_STAGES;
+    uint64_t* chain_empty = chain_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(chain_empty + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.y * GS_TOKENS, n0 = blockIdx.x * tile_n;
+    const int ksplit = gridDim.z;
+    const int all_kb = (K + GS_BK - 1) / GS_BK;
+    const int kb_beg = blockIdx.z * kblocks_per_split;
+    const int n_kb = min(all_kb, kb_beg + kblocks_per_split) - kb_beg;      // at least 1: no split is empty
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GS_STAGES; ++s) {
+            mbar_init(&full[s], GS_WORKERS);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(chain_full, 1);
+        mbar_init(chain_empty, GS_WORKERS);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == GS_WORKERS) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();
+    pdl_wait();
+
+    if (warp < GS_WORKERS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");      // 256 x 232 + 128 x 40 = 384 x 168, what the block was launched with
+        // ---------------- workers.  Task j of a thread: 8 values of k of one row; j 0, 1: A, 2..5: W
+        const int t = threadIdx.x, r0 = t >> 2, ch = t & 3;
+        const float* a_ptr = A + (size_t)min(m0 + r0, M - 1) * lda + ch * 8;
+        const float* a_ptr1 = A + (size_t)min(m0 + r0 + 64, M - 1) * lda + ch * 8;
+        const float* w_ptr[4];
+        uint32_t live = (m0 + r0 < M ? 1u : 0u) | (m0 + r0 + 64 < M ? 2u : 0u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = r0 + 64 * j;
+            w_ptr[j] = W + (size_t)min(n0 + r, N - 1) * ldw + ch * 8;
+            if (r < tile_n && n0 + r < N) live |= 4u << j;
+        }
+        const uint32_t at = (uint32_t)r0 * 64 + (uint32_t)((ch ^ ((r0 >> 1) & 3)) << 4);       // rows 64 on share it: 64 rows are whole swizzle groups
+        float4 x[6][2];
+        auto fetch = [&](int j, int kb) {                  // j a constant: x stays in registers
+            const int k = kb * GS_BK;
+            const float* p = (j == 0 ? a_ptr : j == 1 ? a_ptr1 : w_ptr[(j + 2) & 3]) + k;
+            const bool on = (live >> j) & 1;
+            x[j][0] = on && k + ch * 8 < K ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+            x[j][1] = on && k + ch * 8 + 4 < K ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+
+        const int quad = warp & 3;
+        const int pairs = (tile_n / 16 + 1) / 2, first_pair = warp < 4 ? 0 : (pairs + 1) / 2;
+        const int my_pairs = warp < 4 ? (pairs + 1) / 2 : pairs - first_pair;                  // of 32 features, at most 4
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)first_pair * 32;
+        float acc[4][2][16];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[u][j >> 4][j & 15] = 0.0f;
+        auto add_chain = [&](uint32_t addr) {
+            tc_fence_after();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (u >= my_pairs) break;
+                float v[2][16];
+                tmem_ld32(addr + u * 32, v);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[u][j >> 4][j & 15] += v[j >> 4][j & 15];
+            }
+            tc_fence_before();
+        };
+
+        bool ok = true;
+        int chains = 0;                                    // fetched so far
+#pragma unroll
+        for (int j = 0; j < 6; ++j) fetch(j, kb_beg);
+        for (int i = 0; i < n_kb; ++i) {
+            const int s = i % GS_STAGES;
+            if (i >= GS_STAGES && !MBAR_WAIT(&empty[s], ((uint32_t)(i / GS_STAGES) & 1) ^ 1)) {
+                ok = false;
+                break;
+            }
+            if (i >= GS_CHAIN + 2 && i % GS_CHAIN == 2) {
+                // block i - 3, the chain's last, is done: this wait returns at once
+                if (!MBAR_WAIT(chain_full, (uint32_t)chains & 1)) {
+                    ok = false;
+                    break;
+                }
+                add_chain(lane_addr);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(chain_empty);
+                ++chains;
+            }
+            unsigned char* stage = smem + (size_t)s * GS_STAGE_BYTES;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                if (j >= 2 && (j - 2) * 64 >= tile_n) break;
+                uint4 h, m, l;
+                split_pair(x[j][0].x, x[j][0].y, h.x, m.x, l.x);
+                split_pair(x[j][0].z, x[j][0].w, h.y, m.y, l.y);
+                split_pair(x[j][1].x, x[j][1].y, h.z, m.z, l.z);
+                split_pair(x[j][1].z, x[j][1].w, h.w, m.w, l.w);
+                if (i + 1 < n_kb) fetch(j, kb_beg + i + 1);            // travels while the other tasks are split
+                unsigned char* dst = stage + at + (j < 2 ? j * 64 * 64 : 3 * GS_A_TERM + (j - 2) * 64 * 64);
+                const uint32_t term = j < 2 ? GS_A_TERM : GS_W_TERM;
+                *reinterpret_cast<uint4*>(dst) = h;
+                *reinterpret_cast<uint4*>(dst + term) = m;
+                *reinterpret_cast<uint4*>(dst + 2 * term) = l;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+        const int all_chains = (n_kb + GS_CHAIN - 1) / GS_CHAIN;
+        for (; ok && chains < all_chains; ++chains) {
+            if (!MBAR_WAIT(chain_full, (uint32_t)chains & 1)) {
+                ok = false;
+                break;
+            }
+            add_chain(lane_addr);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(chain_empty);
+        }
+        if (ok) {
+            add_chain(lane_addr + GS_FEATS);               // the second chain: complete with the last block
+        } else if (lane == 0) {
+            atomicOr(status, BFI_STATUS_TIMEOUT);
+        }
+        // every worker is past its last write into the ring, and the products have read it
+        asm volatile("bar.sync 1, %0;" ::"n"(GS_WORKERS * 32) : "memory");
+        float* out = reinterpret_cast<float*>(smem) + (size_t)(quad * 32 + lane) * GS_OUT_LD + first_pair * 32;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (u >= my_pairs) break;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<float4*>(out + u * 32 + j * 4) =
+                    make_float4(acc[u][j >> 2][(j & 3) * 4], acc[u][j >> 2][(j & 3) * 4 + 1], acc[u][j >> 2][(j & 3) * 4 + 2], acc[u][j >> 2][(j & 3) * 4 + 3]);
+        }
+
+        __syncwarp();
+
+        // ---------------- the tile, out as whole rows; with K split, every block finishes a share of the rows
+        gs_meet(ksplit);
+        const int rank = blockIdx.z;                           // the cluster is (1, 1, ksplit)
+        const int per_rank = (GS_TOKENS + ksplit - 1) / ksplit;
+        const int r_beg = rank * per_rank, r_end = min(min(GS_TOKENS, r_beg + per_rank), M - m0);
+        const int quads = tile_n / 4;
+        uint32_t remote[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            remote[r] = smem_u32(smem);
+            if (ksplit > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[r]) : "r"(smem_u32(smem)), "r"(r < ksplit ? r : 0));
+        }
+        for (int idx = threadIdx.x; idx < (r_end - r_beg) * quads; idx += GS_WORKERS * 32) {
+            const int row = r_beg + idx / quads, c = (idx % quads) * 4;
+            const int m = m0 + row, n = n0 + c;
+            if (n >= N) continue;
+            const uint32_t off = ((uint32_t)row * GS_OUT_LD + c) * 4;
+            float v[4];
+            if (ksplit == 1) {
+                const float4 q = *reinterpret_cast<const float4*>(smem + off);
+                v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            } else {
+                float4 q[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    q[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (r < ksplit)
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(q[r].x), "=f"(q[r].y), "=f"(q[r].z), "=f"(q[r].w) : "r"(remote[r] + off));
+                }
+                v[0] = v[1] = v[2] = v[3] = 0.0f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[0] += q[r].x, v[1] += q[r].y, v[2] += q[r].z, v[3] += q[r].w;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < N && !isfinite(v[j])) v[j] = dot_plain(A + (size_t)m * lda, W + (size_t)(n + j) * ldw, K);
+            const bool whole = vec_ok && n + 4 <= N;
+            if (epilogue == EPI_SWIGLU) {
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    if (n + j + 1 >= N) continue;
+                    const float f = gate.in_scale ? gate_in_scale(gate, m, (n + j) >> 1) : 1.0f;
+                    store_from_f32(C, c_dtype, (size_t)m * ldc + ((n + j) >> 1), gate_mul_exact(f * v[j], f * v[j + 1], gate));
+                }
+            } else if (epilogue == EPI_ACCUMULATE) {
+                float* o = reinterpret_cast<float*>(C) + (size_t)m * ldc + n;
+                if (whole) {
+                    const float4 old = *reinterpret_cast<const float4*>(o);
+                    *reinterpret_cast<float4*>(o) = make_float4(old.x + v[0], old.y + v[1], old.z + v[2], old.w + v[3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < N) o[j] += v[j];
+                }
+            } else {
+                if (epilogue == BFI_EPI_RELU_SQUARED) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[j] = relu_squared(v[j]);
+                }
+                if (whole && c_dtype == BFI_F32) {
+                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(C) + (size_t)m * ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < N) store_from_f32(C, c_dtype, (size_t)m * ldc + n + j, v[j]);
+                }
+            }
+        }
+        __syncwarp();
+        gs_meet(ksplit);                                   // no block may leave while another still reads its shared memory
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == GS_WORKERS && lane == 0) {
+            // ---------------- the products
+            const uint32_t idesc = umma_idesc(GS_TOKENS, tile_n);
+            bool ok = true;
+            for (int i = 0; i < n_kb; ++i) {
+                const int s = i % GS_STAGES, chain = i / GS_CHAIN;
+                if (!MBAR_WAIT(&full[s], (uint32_t)(i / GS_STAGES) & 1)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t a = smem_u32(smem + (size_t)s * GS_STAGE_BYTES), w = a + 3 * GS_A_TERM;
+                const uint32_t d2 = tmem_base + GS_FEATS;
+#pragma unroll
+                for (int kk = 0; kk < GS_BK / 16; ++kk) {
+                    const uint64_t ah = umma_desc_sw64(a + kk * 32), am = umma_desc_sw64(a + GS_A_TERM + kk * 32),
+                                   al = umma_desc_sw64(a + 2 * GS_A_TERM + kk * 32);
+                    const uint64_t wh = umma_desc_sw64(w + kk * 32), wm = umma_desc_sw64(w + GS_W_TERM + kk * 32),
+                                   wl = umma_desc_sw64(w + 2 * GS_W_TERM + kk * 32);
+                    umma_bf16(d2, al, wh, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                    umma_bf16(d2, ah, wl, idesc, 1u);
+                    umma_bf16(d2, am, wm, idesc, 1u);
+                    umma_bf16(d2, am, wh, idesc, 1u);
+                    umma_bf16(d2, ah, wm, idesc, 1u);
+                }
+                const bool starts = i % GS_CHAIN == 0;
+                if (starts && chain > 0) {                     // the chain before has been fetched
+                    if (!MBAR_WAIT(chain_empty, (uint32_t)(chain - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                }
+#pragma unroll
+                for (int kk = 0; kk < GS_BK / 16; ++kk)
+                    umma_bf16(tmem_base, umma_desc_sw64(a + kk * 32), umma_desc_sw64(w + kk * 32), idesc, (starts && kk == 0) ? 0u : 1u);
+                umma_commit(&empty[s]);
+                if (i % GS_CHAIN == GS_CHAIN - 1 || i == n_kb - 1) umma_commit(chain_full);
+            }
+            if (!ok) atomicOr(status, BFI_STATUS_TIMEOUT);
+        }
+        __syncwarp();
+        gs_meet(ksplit);
+        gs_meet(ksplit);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == GS_WORKERS) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+    BFI_TRACE_END();
+}
+
+// Reserves the kernel's shared memory; how many clusters of 2 to 8 blocks the GPU holds at once (a cluster lives
+// in one group of SMs, so these are fewer than the SMs divided by its size).  Null after recording an error.
+static const int* gs_clusters() {
+    static int most[9];
+    static const bool ok = [] {
+        cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM);
+        for (int ks = 2; ks <= 8 && e == cudaSuccess; ++ks) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = ks;
+            cfg.gridDim = dim3(1, 1, ks);
+            cfg.blockDim = dim3(GS_THREADS);
+            cfg.dynamicSmemBytes = GS_SMEM;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            e = cudaOccupancyMaxActiveClusters(&most[ks], gemm_split_kernel, &cfg);
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            bfi_fail("gemm_split: cannot reserve %zu bytes of shared memory: %s", GS_SMEM, cudaGetErrorString(e));
+        }
+        return e == cudaSuccess;
+    }();
+    return ok ? most : nullptr;
+}
+
+// Returns 0 on success, 1 on error, 2 when the product is not taken (nothing launched): rows that are not whole
+// 16-byte pieces, sums shorter than GS_MIN_K, and up to 16 rows, which are bound by reading W and belong to the row
+// kernel of gemm_simt.cu.
+// `tune_n`, `tune_split`: the tile's width and the splits of K, for tests and measurements (0: chosen here).
+extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long ldw, void* C, int c_dtype, long ldc, int M, int N, int K,
+                                  int epilogue, int tune_n, int tune_split, int* status, cudaStream_t stream) {
+    BFI_REQUIRE(dtype_ok(c_dtype), "gemm_split: unknown output dtype code %d", c_dtype);
+    BFI_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
+    BFI_REQUIRE(lda >= K && ldw >= K, "gemm_split: a row stride is shorter than K=%d", K);
+    BFI_REQUIRE(epilogue >= 0 && epilogue <= 3, "gemm_split: unknown epilogue %d", epilogue);
+    BFI_REQUIRE(status != nullptr, "gemm_split: a status word is required");
+    if (epilogue == EPI_ACCUMULATE) BFI_REQUIRE(c_dtype == BFI_F32, "gemm_split: accumulation needs a float32 output");
+    if (epilogue == EPI_SWIGLU) {
+        BFI_REQUIRE(N % 2 == 0, "gemm_split: the gated epilogue needs an even N, got %d", N);
+        BFI_REQUIRE(ldc >= N / 2, "gemm_split: output row stride shorter than N/2");
+    } else {
+        BFI_REQUIRE(ldc >= N, "gemm_split: output row stride shorter than N=%d", N);
+    }
+    if (M == 0) return 0;
+    if (M <= 16 || K < GS_MIN_K || K % 4 != 0 || lda % 4 != 0 || ldw % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return 2;
+    const int tiles_m = (M + GS_TOKENS - 1) / GS_TOKENS;
+    if (tiles_m > 65535) return 2;
+
+    // the tile's width and the splits of K that take the least time by an estimate: rounds over the SMs x (blocks
+    // of k x 12 products, which take nearly as long for 128 features as for 256, + what surrounds them)
+    const int kb = (K + GS_BK - 1) / GS_BK, n_sm = bfi_sm_count();
+    const int* clusters = gs_clusters();
+    if (clusters == nullptr) return 1;
+    int tile_n = GS_FEATS, ksplit = 1;
+    double best = -1.0;
+    for (int ks = 1; ks <= 8; ++ks) {
+        if (tune_split > 0 ? ks != tune_split : (ks > 1 && kb / ks < 2 * GS_CHAIN)) continue;
+        for (int tn = GS_FEATS; tn >= 64; tn -= 16) {
+            if (tune_n > 0 && tn != tune_n) continue;
+            const long blocks = (long)tiles_m * ((N + tn - 1) / tn) * ks;
+            const long slots = ks == 1 ? n_sm : (long)clusters[ks] * ks;
+            if (slots < ks) continue;
+            const double cost = (double)((blocks + slots - 1) / slots) * ((double)((kb + ks - 1) / ks) * (1.10 + 0.0026 * tn) + (ks > 1 ? 8.5 : 2.5));
+            if (best < 0.0 || cost < best) best = cost, tile_n = tn, ksplit = ks;
+        }
+    }
+    BFI_REQUIRE(best >= 0.0, "gemm_split: no tile of %d features or no %d splits", tune_n, tune_split);
+    const int per_split = (kb + ksplit - 1) / ksplit;
+    ksplit = (kb + per_split - 1) / per_split;             // no empty splits
+
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((N + tile_n - 1) / tile_n, tiles_m, ksplit);
+    cfg.blockDim = dim3(GS_THREADS);
+    cfg.dynamicSmemBytes = GS_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (ksplit > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = 1;
+        attr[n_attr].val.clusterDim.y = 1;
+        attr[n_attr].val.clusterDim.z = ksplit;
+        ++n_attr;
+    }
+    if (g_bfi_pdl) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    const int vec_ok = (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel, A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split, epilogue, vec_ok,
+                                       g_bfi_gate, status);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return bfi_fail("gemm_split: launch failed: %s", cudaGetErrorString(e));
+    }
+    return bfi_check_launch("gemm_split");
+}
+
+BFI_TRACE_EXPORT(gemm_split)

@@ -9,7 +9,7 @@ import torch
 
 from .library import KernelError, library
 from .ops import (LIGHT_ACT_SILU, _ptr, _rows_2d, _stream, check_memory, check_memory_gates, dtype_code,
-                  rotation_args)
+                  rotation_args, tc_status)
 
 SKINNY_MAX_ROWS = 64
 
@@ -58,19 +58,6 @@ class _SplitScratch:
 
 _split_scratch = _SplitScratch()
 _plan_cache = {}
-
-
-_tc_status = {}
-
-
-def tc_status(device) -> torch.Tensor:
-    """The word in which the tcgen05 kernels record a bounded wait that ran out (bit 8), followed
-    by the prompt attention's two counters (tickets drawn, blocks finished; zero between launches)."""
-    t = _tc_status.get(device)
-    if t is None:
-        t = torch.zeros(4, dtype=torch.int32, device=device)
-        _tc_status[device] = t
-    return t
 
 
 def _check_product(a, w, out, epilogue):

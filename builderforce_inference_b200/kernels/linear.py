@@ -1,8 +1,10 @@
 """``out = a @ w.T`` with a choice of epilogue: the one place that decides which matrix-product
 kernel runs for a shape and a pair of storage types.
 
-* float32 anywhere in the product: the CUDA-core kernels (float32 multiply-add; this is the
-  whole of the 32-bit path, no tensor-core mode is involved);
+* float32 x float32: more than ``SPLIT_MIN_ROWS`` rows run on the tensor cores with every operand split
+  exactly into three bfloat16 terms (closer to the 64-bit product than float32 multiply-adds in
+  a row are); fewer rows, which are bound by reading the weights, run on the CUDA cores (float32 multiply-add);
+* float32 x bfloat16, either way round: the CUDA-core kernels;
 * bfloat16 x bfloat16: few rows stream the weights once through the tensor-core skinny kernel,
   many rows run the tcgen05 kernel; shapes those kernels refuse go to the CUDA-core kernels.
 """
@@ -24,6 +26,7 @@ def _fast_ops():
     return _fast
 
 
+SPLIT_MIN_ROWS = 16                      # the row kernel reads W once for 8 rows and takes up to 16
 GATE_SIGMOID, GATE_GELU_TANH = 0, 1      # kinds of the gated epilogue's activation
 
 
@@ -74,4 +77,6 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 
     if fast:
         if _fast_ops().linear_bf16(a, w, out, epilogue):
             return
+    elif a.dtype == w.dtype and a.shape[0] > SPLIT_MIN_ROWS and ops.gemm_split(a, w, out, epilogue):
+        return
     ops.gemm_simt(a, w, out, epilogue)

@@ -1068,6 +1068,42 @@ def mlstm_step(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, x: torch.
         c_int(dim), c_int(vdim), _stream())
 
 
+_tc_status = {}
+
+
+def tc_status(device) -> torch.Tensor:
+    """The word in which the tcgen05 kernels record a bounded wait that ran out (bit 8), followed
+    by the prompt attention's two counters (tickets drawn, blocks finished; zero between launches)."""
+    t = _tc_status.get(device)
+    if t is None:
+        t = torch.zeros(4, dtype=torch.int32, device=device)
+        _tc_status[device] = t
+    return t
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, tile_n: int = 0, splits: int = 0) -> bool:
+    """``out = a @ w.T`` for float32 operands on the tensor cores, every operand split exactly into three bfloat16
+    terms.  False for products it does not take (up to 16 rows; sums shorter than 512; rows that are not whole 16-byte pieces).
+    ``tile_n``, ``splits``: the tile's width and the splits of K, for tests and measurements (0: the kernel's choice)."""
+    _need_cuda(a, w, out)
+    _rows_2d(a, "A")
+    _rows_2d(w, "W")
+    _rows_2d(out, "C")
+    m, k = a.shape
+    n = w.shape[0]
+    if a.dtype != torch.float32 or w.dtype != torch.float32:
+        return False
+    if w.shape[1] != k:
+        raise KernelError(f"matrix product: A is {tuple(a.shape)} but W is {tuple(w.shape)}")
+    cols = n // 2 if epilogue == EPI_SWIGLU else n
+    if out.shape != (m, cols):
+        raise KernelError(f"matrix product: output must be [{m}, {cols}], got {tuple(out.shape)}")
+    return library("core").call_optional(
+        "bfi_gemm_split_f32", _ptr(a), c_long(a.stride(0)), _ptr(w), c_long(w.stride(0)), _ptr(out), c_int(dtype_code(out.dtype)),
+        c_long(out.stride(0)), c_int(m), c_int(n), c_int(k), c_int(epilogue), c_int(tile_n), c_int(splits), _ptr(tc_status(a.device)),
+        _stream())
+
+
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE) -> None:
     """``out = a @ w.T`` on the CUDA cores in float32 arithmetic (any dtypes, any sizes)."""
     _need_cuda(a, w, out)

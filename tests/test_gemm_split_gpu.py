@@ -1,0 +1,83 @@
+"""The float32 product on the tensor cores (three bfloat16 terms per operand) against a 64-bit product, at the edges of
+its tiles, chains and splits, and beside the CUDA-core kernel on the same data."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def operands(m, n, k, seed, wide=False):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    a = torch.randn(m, k, generator=g, device=DEV)
+    w = torch.randn(n, k, generator=g, device=DEV) * k ** -0.5
+    if wide:        # magnitudes over many powers of two: the lower terms of large values meet the upper ones of small
+        a *= torch.exp(3 * torch.randn(m, k, generator=g, device=DEV))
+    return a, w
+
+
+def err(x, ref):
+    return float((x.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("m,n,k,tile_n,splits", [
+    (17, 64, 512, 0, 0), (127, 250, 516, 0, 0), (128, 256, 512, 256, 1), (129, 257, 516, 256, 1), (300, 1000, 1000, 208, 2),
+    (40, 330, 2560, 64, 8), (65, 96, 1284, 80, 3), (256, 512, 1152, 144, 5), (513, 2000, 2728, 0, 0)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_product_is_no_further_off_than_multiply_adds(m, n, k, tile_n, splits, wide):
+    from builderforce_inference_b200.kernels import ops
+    a, w = operands(m, n, k, m + n + k, wide)
+    ref = a.double() @ w.double().T
+    plain, out = torch.empty(m, n, device=DEV), torch.full((m, n + 4), 7.0, device=DEV)
+    ops.gemm_simt(a, w, plain)
+    assert ops.gemm_split(a, w, out[:, :n], ops.EPI_STORE, tile_n, splits)
+    assert int(ops.tc_status(DEV)[0].item()) == 0
+    assert torch.all(out[:, n:] == 7.0)
+    # one chain of 128 products truncates eight times (2^-23 of the running sum each at most), rounded sums follow
+    assert err(out[:, :n], ref) < 3e-7
+    assert err(out[:, :n], ref) <= err(plain, ref)
+
+
+@pytest.mark.parametrize("splits", [1, 4])
+def test_epilogues_strides_and_output_types(splits):
+    from builderforce_inference_b200.kernels import ops
+    m, n, k = 70, 328, 1024
+    a, w = operands(m, n, k, 5)
+    big = torch.zeros(m, k + 12, device=DEV)
+    big[:, 4:4 + k] = a
+    a = big[:, 4:4 + k]
+    ref = a.double() @ w.double().T
+    old = torch.randn(m, n, device=DEV)
+    out = old.clone()
+    assert ops.gemm_split(a, w, out, ops.EPI_ACCUMULATE, 0, splits) and err(out, ref + old.double()) < 3e-7
+    out = torch.empty(m, n // 2 + 1, device=DEV)[:, :n // 2]               # rows that are no whole 16-byte pieces
+    assert ops.gemm_split(a, w, out, ops.EPI_SWIGLU, 0, splits)
+    assert err(out, torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]) < 6e-7
+    out = torch.empty(m, n, device=DEV)
+    assert ops.gemm_split(a, w, out, ops.EPI_RELU_SQUARED, 0, splits) and err(out, ref.clamp(min=0).square()) < 6e-7
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    assert ops.gemm_split(a, w, out, ops.EPI_STORE, 0, splits) and err(out, ref) < 2.0 ** -8
+
+
+def test_results_that_are_not_finite_come_out_as_multiply_adds_give_them():
+    from builderforce_inference_b200.kernels import ops
+    a, w = operands(40, 80, 512, 6)
+    w[:, 7] = 1.0                                   # its lower terms are zero: zero times infinity must not show
+    a[3, 7], a[5, 9], a[6, 0] = float("inf"), float("nan"), 3.4e38         # the last rounds to infinity in bfloat16
+    w[10, 0], w[11, 0] = 0.5, 4.0
+    plain, out = torch.empty(40, 80, device=DEV), torch.empty(40, 80, device=DEV)
+    ops.gemm_simt(a, w, plain)
+    assert ops.gemm_split(a, w, out)
+    assert torch.equal(torch.isnan(out), torch.isnan(plain)) and torch.equal(torch.isinf(out), torch.isinf(plain))
+    assert torch.equal(out[3], plain[3]) and torch.equal(out[6, 10:12], plain[6, 10:12])
+
+
+@pytest.mark.parametrize("m,n,k", [(16, 64, 512), (20, 64, 515), (20, 64, 508)])
+def test_what_it_leaves_to_the_other_kernels(m, n, k):
+    from builderforce_inference_b200.kernels import ops
+    from builderforce_inference_b200.kernels.linear import linear
+    a, w = operands(m, n, k, 7)
+    out = torch.empty(m, n, device=DEV)
+    assert not ops.gemm_split(a, w, out)
+    linear(a, w, out)
+    assert err(out, a.double() @ w.double().T) < 1e-6
