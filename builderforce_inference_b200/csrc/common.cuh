@@ -131,6 +131,21 @@ __device__ __forceinline__ void store_from_f32(void* p, int dtype, size_t i, flo
         reinterpret_cast<bf16*>(p)[i] = __float2bfloat16_rn(v);
 }
 
+// A float32 value is the sum of three bfloat16 ones, exactly: each is the rounding of what those before it leave
+// (8 significant bits each).  The terms h, m and l of two values, packed in pairs.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    h = *reinterpret_cast<uint32_t*>(&t);
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xffff0000u);
+    t = __floats2bfloat162_rn(a, b);
+    m = *reinterpret_cast<uint32_t*>(&t);
+    a -= __uint_as_float(m << 16);
+    b -= __uint_as_float(m & 0xffff0000u);
+    t = __floats2bfloat162_rn(a, b);
+    l = *reinterpret_cast<uint32_t*>(&t);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -1,0 +1,608 @@
+// The recurrences of recurrence.cu over runs of new tokens, on the tensor cores: bfloat16 q, k, v, float32 state and
+// arithmetic.  A sequence is cut into chunks of 64 tokens that run side by side, in three launches: what every
+// chunk adds to the state; the chunks of a sequence in order (the state each starts from); the outputs.  With
+// positions inside the chunk, w_tj the product of the decays of tokens j+1 .. t and S the state before the chunk:
+//     adds   U   = sum_j (k_j w_nj) (c_j v_j)^T
+//     out    o_t = (q_t w_t0)^T S + sum_{j <= t} (sum_d q_t w_tj k_j) c_j v_j + skip v_t
+// Nothing is rounded to 16 bits on the way: q, k and v are bfloat16 as they come, and every float32 operand of a
+// tensor-core product (S, the decayed scores, decayed keys, queries and values) is split exactly into three
+// bfloat16 terms, of whose products all that reach 2^-18 of the whole are taken; the products of the first terms
+// have chains of sums of their own, four or eight instructions long, so the tensor cores' truncation stays at the level
+// of float32 rounding.
+//   one decay per head: log decays are summed in 64 bits and w is the exponential of a difference;
+//   a decay per row:    with E_t the product of the chunk's decays up to t, w_tj = E_t (1 / E_j): the queries carry E_t
+//                       and the keys 1 / E_j, as long as E stays above 2^-80 in every row.
+// A chunk in which it does not, or that holds a value which is not finite, is walked token by token in float32 by the
+// same block (plain_chunk), as recurrence.cu would.
+//
+// Work split: a block per (head, up to 128 columns, chunk); a warp owns 16 columns (with fewer columns, or sixteen
+// warps, the warps share the rows) and splits its B operands (S, c v) in registers, straight from where they lie.
+//
+// What bounds it: the latency chain of a block's phases (pieces, decays, scores, outputs) with 16 warps on an SM, and the
+// scratch (D x V floats per chunk and head: written, read and rewritten, read), which stays in L2 for prompts of a few
+// thousand tokens.  Measured, recurrence.cu -> these kernels (heads of 128 x 128; a walk in order takes 1.4 us a token):
+//     32 heads, one prompt of 2,048 tokens, a decay per head: 757 -> 119 us; per row: 770 -> 233 us
+//     16 heads, prompts of 1,500, 1,043, 587 and 130 tokens, a decay per row: 548 -> 210 us
+//     16 heads, 8 prompts of 33 to 500 tokens, a decay per head: 360 -> 74 us
+// Distance from a 64-bit walk, relative to the 2-norm (2,048 tokens; a float32 walk in order in brackets): outputs 1.3e-7
+// (1.8e-7), state 0.9e-7 (1.5e-7); a decay per row: 1.9e-7 (2.1e-7), 1.7e-7 (1.8e-7).
+#include "chunk_tiles.cuh"
+
+#define DC_LEN 64            // tokens per chunk
+#define DC_STEP 1            // REC_DECAY_STEP and REC_DECAY_SIGMOID of recurrence.cu
+#define DC_SIGMOID 2
+#define DC_LDP (DC_LEN + 8)
+#define DC_SMALLEST 8.2718061255302767e-25f      // 2^-80
+// Warps of a block: eight, two blocks on an SM; sixteen where three terms of queries and keys leave room for one block
+static __host__ __device__ constexpr int dc_warps(int mode, bool out) { return mode == DC_SIGMOID && out ? 16 : 8; }
+
+struct DcArgs {
+    long qk_stride, v_stride, r_stride, out_stride;
+    int q_off, k_off, v_off, r_off;
+    int H, D, V, heads_per_group, v_blocks;
+    float q_scale, inv_tau;
+    const float *bias, *rate, *skip;
+    const int *cu_seqlens, *seq_slot;
+};
+
+__device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
+__device__ __forceinline__ float dc_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
+// any of eight bfloat16 values infinite or NaN
+__device__ __forceinline__ bool dc_not_finite(uint4 x) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bad |= (w[i] & 0x7f80u) == 0x7f80u || (w[i] & 0x7f800000u) == 0x7f800000u;
+    return bad;
+}
+
+struct DcSmem {
+    int ldq, ldv, lde;
+    size_t q, k, v, p, e, tot, cum, c, w, total;      // p and e share their place: e is dead when p is made
+};
+// `out`: the layout of the kernel that makes the outputs; otherwise of the one that makes what a chunk adds.
+static __host__ __device__ inline DcSmem dc_layout(int D, int VB, bool sigmoid, bool out) {
+    DcSmem s;
+    s.ldq = D + 8, s.ldv = VB + 8, s.lde = D + 4;
+    const size_t terms = sigmoid ? 3 : 1;
+    size_t o = 0;
+    auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 127) / 128 * 128; return at; };
+    s.q = take(out ? terms * DC_LEN * s.ldq * 2 : 0);
+    s.k = take(terms * DC_LEN * s.ldq * 2);
+    s.v = take((size_t)DC_LEN * s.ldv * 2);
+    const size_t p = out ? (size_t)3 * DC_LEN * DC_LDP * 2 : 0, e = sigmoid ? (size_t)DC_LEN * s.lde * 4 : 0;
+    s.p = s.e = take(p > e ? p : e);
+    s.tot = take(sigmoid ? (size_t)2 * D * 4 : 4);
+    s.cum = take((size_t)DC_LEN * 8);
+    s.c = take((size_t)DC_LEN * 4);
+    s.w = take((size_t)DC_LEN * 4);
+    const size_t plain = ((size_t)D * VB + 3 * D + 512 + 8) * 4;      // plain_chunk: state, q, k, a, sums
+    s.total = o > plain ? o : plain;
+    return s;
+}
+
+// A chunk token by token in float32 multiply-adds.  OUT: from the state `start`, writing outputs; otherwise from zero,
+// leaving the state it ends with in `add` and the product of its decays in `decays`.
+template <int MODE, bool OUT>
+__device__ __noinline__ void plain_chunk(float* sm, const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, const bf16* __restrict__ raw,
+                                         float* __restrict__ out, const float* start, float* add, float* __restrict__ decays,
+                                         const DcArgs& a, int h, int v0, int t0, int n) {
+    constexpr int THREADS = dc_warps(MODE, OUT) * 32;
+    const int D = a.D, VB = min(128, a.V - v0), tid = threadIdx.x;
+    float* S = sm;
+    float *qs = S + (size_t)D * VB, *ks = qs + D, *as = ks + D, *red = as + D, *step = red + THREADS;
+    const int c = tid % VB, g = tid / VB, ng = THREADS / VB;
+    const int grp = h / a.heads_per_group;
+    const float skip = a.skip ? a.skip[h] : 0.0f;
+    float prod = 1.0f;
+    __syncthreads();
+    for (int i = tid; i < D * VB; i += THREADS) S[i] = OUT ? start[(size_t)(i / VB) * a.V + i % VB] : 0.0f;
+    for (int t = 0; t < n; ++t) {
+        const size_t tok = (size_t)t0 + t;
+        __syncthreads();
+        if (tid == 0) *step = MODE == DC_STEP ? dc_softplus(to_f32(raw[tok * a.r_stride + a.r_off + h]) + a.bias[h]) : 1.0f;
+        __syncthreads();
+        if (tid < D) {
+            const float w = MODE == DC_STEP ? expf(-a.rate[h] * *step)
+                                            : expf(dc_log_sigmoid(to_f32(raw[tok * a.r_stride + a.r_off + (size_t)h * D + tid]) +
+                                                                  a.bias[(size_t)h * D + tid]) * a.inv_tau);
+            qs[tid] = OUT ? to_f32(qk[tok * a.qk_stride + a.q_off + (size_t)grp * D + tid]) * a.q_scale : 0.0f;
+            ks[tid] = to_f32(qk[tok * a.qk_stride + a.k_off + (size_t)grp * D + tid]);
+            as[tid] = w;
+            prod *= w;
+        }
+        __syncthreads();
+        const float vv = to_f32(vsrc[tok * a.v_stride + a.v_off + (size_t)h * a.V + v0 + c]);
+        float acc = 0.0f;
+        if (g < ng) {
+            for (int d = g; d < D; d += ng) {
+                const float s = fmaf(as[d], S[d * VB + c], ks[d] * (*step * vv));
+                S[d * VB + c] = s;
+                if (OUT) acc = fmaf(s, qs[d], acc);
+            }
+        }
+        red[tid] = acc;
+        __syncthreads();
+        if (OUT && tid < VB) {
+            float o = 0.0f;
+            for (int i = 0; i < ng; ++i) o += red[i * VB + tid];
+            out[tok * a.out_stride + (size_t)h * a.V + v0 + c] = fmaf(skip, vv, o);
+        }
+    }
+    __syncthreads();
+    if (!OUT) {
+        for (int i = tid; i < D * VB; i += THREADS) add[(size_t)(i / VB) * a.V + i % VB] = S[i];
+        if (v0 == 0 && tid < D) decays[tid] = prod;
+    }
+}
+
+__device__ __forceinline__ void dc_put_terms(bf16* dst, int term, const float (&x)[8]) {
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split_pair(x[2 * j], x[2 * j + 1], h[j], m[j], l[j]);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(dst + term) = make_uint4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<uint4*>(dst + 2 * term) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// OUT false: what a chunk adds, and the product of its decays per row.  OUT true: its outputs, from the state it starts from.
+// DMAX: the head's rows, a multiple of 16, are at most this (64 or 128).
+template <int MODE, bool OUT, int DMAX>
+__global__ void __launch_bounds__(dc_warps(MODE, OUT) * 32)
+decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, const bf16* __restrict__ raw, float* __restrict__ out,
+                   float* __restrict__ chunk_state, float* __restrict__ chunk_decay, const DcArgs a) {
+    constexpr int WARPS = dc_warps(MODE, OUT), THREADS = WARPS * 32;
+    pdl_trigger();
+    extern __shared__ __align__(128) unsigned char dc_smem[];
+    const int seq = blockIdx.y;
+    if (a.seq_slot[seq] < 0) return;
+    const int D = a.D, V = a.V, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x / a.v_blocks;
+    const int v0 = (blockIdx.x - h * a.v_blocks) * 128, VB = min(128, V - v0);
+    const int first = blockIdx.z * DC_LEN;
+    const int nt = a.cu_seqlens[seq + 1] - a.cu_seqlens[seq];
+    if (first >= nt) return;
+    size_t no = blockIdx.z;                              // the chunk's running number
+    for (int s = 0; s < seq; ++s) no += (a.cu_seqlens[s + 1] - a.cu_seqlens[s] + DC_LEN - 1) / DC_LEN;
+    const int t0 = a.cu_seqlens[seq] + first, n = min(DC_LEN, nt - first);
+    const int grp = h / a.heads_per_group;
+    const DcSmem L = dc_layout(D, VB, MODE == DC_SIGMOID, OUT);
+    bf16* Qs = reinterpret_cast<bf16*>(dc_smem + L.q);
+    bf16* Ks = reinterpret_cast<bf16*>(dc_smem + L.k);
+    bf16* Vs = reinterpret_cast<bf16*>(dc_smem + L.v);
+    bf16* Ps = reinterpret_cast<bf16*>(dc_smem + L.p);
+    float* Es = reinterpret_cast<float*>(dc_smem + L.e);
+    float* tot = reinterpret_cast<float*>(dc_smem + L.tot);
+    double* cum = reinterpret_cast<double*>(dc_smem + L.cum);
+    float* cs = reinterpret_cast<float*>(dc_smem + L.c);
+    float* ws = reinterpret_cast<float*>(dc_smem + L.w);
+    const int q_term = DC_LEN * L.ldq, p_term = DC_LEN * DC_LDP;
+    float* my_state = chunk_state + (no * a.H + h) * (size_t)D * V + v0;
+    float* my_decay = chunk_decay + (no * a.H + h) * (size_t)D;
+    pdl_wait();
+
+    // ---- q, k, v and the decays into shared memory: a thread's 16-byte pieces are all asked for before the first is used
+    bool bad = false;
+    const int D8 = D >> 3, V8 = VB >> 3;
+    constexpr int NP = (DC_LEN * (DMAX / 8) + THREADS - 1) / THREADS, NV = DC_LEN * 16 / THREADS;
+    uint4 xq[NP], xk[NP], xr[NP], xv[NV];
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < NP; ++u) {
+        const int i = tid + u * THREADS, t = i / D8, e = i - t * D8;
+        xq[u] = xk[u] = xr[u] = zero;
+        if (t < n) {
+            const bf16* row = qk + (size_t)(t0 + t) * a.qk_stride + (size_t)grp * D + e * 8;
+            if (MODE == DC_SIGMOID) xr[u] = *reinterpret_cast<const uint4*>(raw + (size_t)(t0 + t) * a.r_stride + a.r_off + (size_t)h * D + e * 8);
+            if (OUT) xq[u] = *reinterpret_cast<const uint4*>(row + a.q_off);
+            xk[u] = *reinterpret_cast<const uint4*>(row + a.k_off);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        const int i = tid + u * THREADS, t = i / V8, e = i - t * V8;
+        xv[u] = zero;
+        if (t < n) xv[u] = *reinterpret_cast<const uint4*>(vsrc + (size_t)(t0 + t) * a.v_stride + a.v_off + (size_t)h * V + v0 + e * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < NP; ++u) bad |= dc_not_finite(xq[u]) || dc_not_finite(xk[u]);
+#pragma unroll
+    for (int u = 0; u < NV; ++u) bad |= dc_not_finite(xv[u]);
+    if (MODE == DC_STEP) {
+        if (warp == 0) {                                 // log decays summed over the chunk: two tokens a lane
+            float c2[2];
+            double l2[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = 2 * lane + i;
+                c2[i] = t < n ? dc_softplus(to_f32(raw[(size_t)(t0 + t) * a.r_stride + a.r_off + h]) + a.bias[h]) : 0.0f;
+                l2[i] = t < n ? (double)(-a.rate[h] * c2[i]) : 0.0;
+            }
+            double run = l2[0] + l2[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double up = __shfl_up_sync(0xffffffffu, run, o);
+                if (lane >= o) run += up;
+            }
+            const double all = __shfl_sync(0xffffffffu, run, 31);
+            bad |= !(all > -1e30);                       // an infinite step leaves no difference to take
+            cum[2 * lane] = run - l2[1], cum[2 * lane + 1] = run;
+            cs[2 * lane] = c2[0], cs[2 * lane + 1] = c2[1];
+            if (OUT) {
+                ws[2 * lane] = expf((float)cum[2 * lane]) * a.q_scale, ws[2 * lane + 1] = expf((float)run) * a.q_scale;
+            } else {
+                ws[2 * lane] = c2[0] * expf((float)(all - cum[2 * lane])), ws[2 * lane + 1] = c2[1] * expf((float)(all - run));
+                if (lane == 0) tot[0] = expf((float)all);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int i = tid + u * THREADS, t = i / D8, e = i - t * D8;
+            if (t >= DC_LEN) continue;
+            if (OUT) *reinterpret_cast<uint4*>(Qs + t * L.ldq + e * 8) = xq[u];
+            *reinterpret_cast<uint4*>(Ks + t * L.ldq + e * 8) = xk[u];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int i = tid + u * THREADS, t = i / D8, e = i - t * D8;
+            if (t >= DC_LEN) continue;
+            const float* b = a.bias + (size_t)h * D + e * 8;
+            const float4 b0 = *reinterpret_cast<const float4*>(b), b1 = *reinterpret_cast<const float4*>(b + 4);
+            const float b8[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            const uint32_t r4[4] = {xr[u].x, xr[u].y, xr[u].z, xr[u].w};
+            float w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                w[j] = t < n ? expf(dc_log_sigmoid((j & 1 ? bf16_hi(r4[j >> 1]) : bf16_lo(r4[j >> 1])) + b8[j]) * a.inv_tau) : 1.0f;
+            float* dst = Es + t * L.lde + e * 8;
+            *reinterpret_cast<float4*>(dst) = make_float4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<float4*>(dst + 4) = make_float4(w[4], w[5], w[6], w[7]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        const int i = tid + u * THREADS, t = i / V8, e = i - t * V8;
+        if (t < DC_LEN) *reinterpret_cast<uint4*>(Vs + t * L.ldv + e * 8) = xv[u];
+    }
+    if (MODE == DC_SIGMOID) {
+        __syncthreads();
+        // products along the tokens, in two halves of the chunk: from the start (OUT: up to and with t) or from
+        // the end (after t)
+        for (int i = tid; i < 2 * D; i += THREADS) {
+            const int half = i / D, d = i - half * D;
+            float p = 1.0f;
+#pragma unroll 8
+            for (int j = 0; j < DC_LEN / 2; ++j) {
+                const int t = half * (DC_LEN / 2) + (OUT ? j : DC_LEN / 2 - 1 - j);
+                const float w = Es[t * L.lde + d];
+                if (OUT) p *= w;
+                Es[t * L.lde + d] = p;
+                if (!OUT) p *= w;
+            }
+            tot[i] = p;
+        }
+        __syncthreads();
+        if (OUT)
+            for (int d = tid; d < D; d += THREADS) bad |= !(tot[d] * tot[D + d] >= DC_SMALLEST);
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int i = tid + u * THREADS, t = i / D8, e = i - t * D8;
+            if (t >= DC_LEN) continue;
+            float E[8], x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                E[j] = Es[t * L.lde + e * 8 + j];
+                if (OUT ? t >= DC_LEN / 2 : t < DC_LEN / 2) E[j] *= tot[(OUT ? 0 : D) + e * 8 + j];
+            }
+            const uint32_t q4[4] = {xq[u].x, xq[u].y, xq[u].z, xq[u].w}, k4[4] = {xk[u].x, xk[u].y, xk[u].z, xk[u].w};
+            if (OUT) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = (j & 1 ? bf16_hi(q4[j >> 1]) : bf16_lo(q4[j >> 1])) * E[j];
+                dc_put_terms(Qs + t * L.ldq + e * 8, q_term, x);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                x[j] = j & 1 ? bf16_hi(k4[j >> 1]) : bf16_lo(k4[j >> 1]);
+                x[j] = OUT ? x[j] / E[j] : x[j] * E[j];
+            }
+            dc_put_terms(Ks + t * L.ldq + e * 8, q_term, x);
+        }
+    }
+    if (__syncthreads_or(bad)) {
+        plain_chunk<MODE, OUT>(reinterpret_cast<float*>(dc_smem), qk, vsrc, raw, out, my_state, my_state, my_decay, a, h, v0, t0, n);
+        return;
+    }
+
+    // ---- a warp's columns: 16 of them, and a share of the rows where there are more warps than columns
+    const int across = VB > 64 ? 8 : (VB > 32 ? 4 : (VB > 16 ? 2 : 1));        // warps side by side
+    const int vt = warp & (across - 1), mine = warp / across, share = WARPS / across;
+    const bool has_columns = vt * 16 < VB;
+    const int g = lane >> 2, t2 = (lane & 3) * 2;
+
+    if (!OUT) {
+        if (v0 == 0)
+            for (int d = tid; d < D; d += THREADS) my_decay[d] = MODE == DC_STEP ? tot[0] : tot[d] * tot[D + d];
+        if (!has_columns) return;
+        constexpr int BT = MODE == DC_STEP ? 3 : 1;      // terms of (c v); v itself is one
+        uint32_t b[4][BT][4];
+#pragma unroll
+        for (int kj = 0; kj < 4; ++kj) {
+            uint32_t raw4[4];
+            lc_b_rows(raw4, Vs + kj * 16 * L.ldv + vt * 16, L.ldv);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int j = kj * 16 + t2 + (i & 1) * 8;
+                if (MODE == DC_STEP)
+                    split_pair(bf16_lo(raw4[i]) * ws[j], bf16_hi(raw4[i]) * ws[j + 1], b[kj][0][i], b[kj][BT > 1 ? 1 : 0][i], b[kj][BT > 2 ? 2 : 0][i]);
+                else
+                    b[kj][0][i] = raw4[i];
+            }
+        }
+#pragma unroll 2
+        for (int td = mine; td < D / 16; td += share) {
+            float hi[2][4] = {}, lo[2][4] = {};
+#pragma unroll
+            for (int kj = 0; kj < 4; ++kj) {
+                uint32_t fa[4];
+                lc_a_cols(fa, Ks + kj * 16 * L.ldq + td * 16, L.ldq);          // A[m = d][k = j] = k_j[d]
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma16816(hi[nb], fa, b[kj][0][2 * nb], b[kj][0][2 * nb + 1]);
+#pragma unroll
+                for (int x = 2; x >= 1; --x) {
+                    if (MODE == DC_SIGMOID) lc_a_cols(fa, Ks + x * q_term + kj * 16 * L.ldq + td * 16, L.ldq);
+                    const int xb = x < BT ? x : 0;
+#pragma unroll
+                    for (int nb = 0; nb < 2; ++nb) mma16816(lo[nb], fa, b[kj][xb][2 * nb], b[kj][xb][2 * nb + 1]);
+                }
+            }
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+                float* dst = my_state + (size_t)(td * 16 + g) * V + vt * 16 + nb * 8 + t2;
+                *reinterpret_cast<float2*>(dst) = make_float2(hi[nb][0] + lo[nb][0], hi[nb][1] + lo[nb][1]);
+                *reinterpret_cast<float2*>(dst + (size_t)8 * V) = make_float2(hi[nb][2] + lo[nb][2], hi[nb][3] + lo[nb][3]);
+            }
+        }
+        return;
+    }
+
+    // the state's rows as they become B operands, asked for AHEAD steps of 16 before their turn: the first while the
+    // scores are made
+    constexpr int AHEAD = 2;
+    const float* sp = my_state + (size_t)t2 * V + vt * 16 + g;
+    float s[AHEAD][8];
+    auto fetch_state = [&](int kk, float (&x)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = sp[(size_t)(kk * 16 + (i & 1) + ((i >> 1) & 1) * 8) * V + (i >> 2) * 8];
+    };
+    if (has_columns) {
+#pragma unroll
+        for (int kk = 0; kk < AHEAD; ++kk)
+            if (kk * 16 < D) fetch_state(kk, s[kk]);
+    }
+
+    // ---- scores of the 16x16 tiles at or below the diagonal, decayed, and their terms
+    for (int job = warp; job < 10; job += WARPS) {
+        int ti = 0, tj = job;
+        while (tj > ti) tj -= ++ti;                      // job -> (ti, tj) with tj <= ti
+        float hi[2][2][4] = {}, lo[2][4] = {};           // the first terms' products: two chains of at most four
+#pragma unroll
+        for (int kk = 0; kk < DMAX / 16; ++kk) {
+            if (kk * 16 >= D) break;
+            uint32_t fa[4], fb[4];
+            const bf16 *qt = Qs + ti * 16 * L.ldq + kk * 16, *kt = Ks + tj * 16 * L.ldq + kk * 16;
+            lc_a_rows(fa, qt, L.ldq);
+            lc_b_cols(fb, kt, L.ldq);
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) mma16816(hi[kk & 1][nb], fa, fb[2 * nb], fb[2 * nb + 1]);
+            if (MODE == DC_SIGMOID) {
+                uint32_t fm[4], fl[4], x[4];
+                lc_a_rows(fm, qt + q_term, L.ldq);
+                lc_a_rows(fl, qt + 2 * q_term, L.ldq);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma16816(lo[nb], fl, fb[2 * nb], fb[2 * nb + 1]), mma16816(lo[nb], fm, fb[2 * nb], fb[2 * nb + 1]);
+                lc_b_cols(x, kt + q_term, L.ldq);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma16816(lo[nb], fm, x[2 * nb], x[2 * nb + 1]), mma16816(lo[nb], fa, x[2 * nb], x[2 * nb + 1]);
+                lc_b_cols(x, kt + 2 * q_term, L.ldq);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma16816(lo[nb], fa, x[2 * nb], x[2 * nb + 1]);
+            }
+        }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = ti * 16 + g + r * 8, j = tj * 16 + nb * 8 + t2;
+                float x[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float f = a.q_scale;
+                    if (MODE == DC_STEP) f *= cs[j + i] * expf((float)(cum[t] - cum[min(j + i, t)]));
+                    x[i] = j + i <= t ? ((hi[0][nb][2 * r + i] + hi[1][nb][2 * r + i]) + lo[nb][2 * r + i]) * f : 0.0f;
+                }
+                uint32_t th, tm, tl;
+                split_pair(x[0], x[1], th, tm, tl);
+                uint32_t* dst = reinterpret_cast<uint32_t*>(Ps + t * DC_LDP + j);
+                dst[0] = th, dst[p_term / 2] = tm, dst[p_term] = tl;
+            }
+    }
+    __syncthreads();
+    if (!has_columns) return;
+
+    // ---- the state's part; with a decay per row, whose operands have roundings of their own, the first terms' chain is cut
+    // in the middle
+    constexpr int NT = 32 / WARPS;                       // groups of 16 tokens of a warp at most: mine, mine + share, ...
+    constexpr int CUT = MODE == DC_SIGMOID ? 4 : 1 << 20;
+    float hi[4][2][4] = {}, cut[4][2][4] = {}, lo[4][2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < DMAX / 16; ++kk) {
+        if (kk * 16 >= D) break;
+        uint32_t bh[4], bm[4], bl[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split_pair(s[kk % AHEAD][2 * i], s[kk % AHEAD][2 * i + 1], bh[i], bm[i], bl[i]);
+        if ((kk + AHEAD) * 16 < D) fetch_state(kk + AHEAD, s[kk % AHEAD]);
+        if (kk == CUT) {
+#pragma unroll
+            for (int u = 0; u < NT; ++u)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) cut[u][i >> 2][i & 3] = hi[u][i >> 2][i & 3], hi[u][i >> 2][i & 3] = 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < NT; ++u) {
+            const int ti = mine + u * share;
+            if (ti >= 4) break;
+            const bf16* qt = Qs + ti * 16 * L.ldq + kk * 16;
+            uint32_t fa[4];
+            lc_a_rows(fa, qt, L.ldq);
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+                mma16816(hi[u][nb], fa, bh[2 * nb], bh[2 * nb + 1]);
+                mma16816(lo[u][nb], fa, bl[2 * nb], bl[2 * nb + 1]);
+                mma16816(lo[u][nb], fa, bm[2 * nb], bm[2 * nb + 1]);
+            }
+            if (MODE == DC_SIGMOID) {
+                lc_a_rows(fa, qt + q_term, L.ldq);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) {
+                    mma16816(lo[u][nb], fa, bm[2 * nb], bm[2 * nb + 1]);
+                    mma16816(lo[u][nb], fa, bh[2 * nb], bh[2 * nb + 1]);
+                }
+                lc_a_rows(fa, qt + 2 * q_term, L.ldq);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma16816(lo[u][nb], fa, bh[2 * nb], bh[2 * nb + 1]);
+            }
+        }
+    }
+    // ---- the chunk's own part
+    const float skip = a.skip ? a.skip[h] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+        const int ti = mine + u * share;
+        if (ti >= 4) break;
+        float ph[2][4] = {}, pl[2][4] = {};
+#pragma unroll
+        for (int kj = 0; kj < 4; ++kj) {
+            if (kj > ti) break;
+            uint32_t fa[4], fb[4];
+            lc_b_rows(fb, Vs + kj * 16 * L.ldv + vt * 16, L.ldv);
+            const bf16* pt = Ps + ti * 16 * DC_LDP + kj * 16;
+            lc_a_rows(fa, pt, DC_LDP);
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) mma16816(ph[nb], fa, fb[2 * nb], fb[2 * nb + 1]);
+            lc_a_rows(fa, pt + 2 * p_term, DC_LDP);
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) mma16816(pl[nb], fa, fb[2 * nb], fb[2 * nb + 1]);
+            lc_a_rows(fa, pt + p_term, DC_LDP);
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) mma16816(pl[nb], fa, fb[2 * nb], fb[2 * nb + 1]);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int t = ti * 16 + g + r * 8;
+            if (t >= n) continue;
+            const float f = MODE == DC_STEP ? ws[t] : a.q_scale;
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+                const uint32_t v2 = *reinterpret_cast<const uint32_t*>(Vs + t * L.ldv + vt * 16 + nb * 8 + t2);
+                float2 o;
+                o.x = fmaf((cut[u][nb][2 * r] + hi[u][nb][2 * r]) + lo[u][nb][2 * r], f, fmaf(skip, bf16_lo(v2), ph[nb][2 * r] + pl[nb][2 * r]));
+                o.y = fmaf((cut[u][nb][2 * r + 1] + hi[u][nb][2 * r + 1]) + lo[u][nb][2 * r + 1], f,
+                           fmaf(skip, bf16_hi(v2), ph[nb][2 * r + 1] + pl[nb][2 * r + 1]));
+                *reinterpret_cast<float2*>(out + (size_t)(t0 + t) * a.out_stride + (size_t)h * V + v0 + vt * 16 + nb * 8 + t2) = o;
+            }
+        }
+    }
+}
+
+// One thread per four elements of a head's state: every chunk's place receives the state the chunk starts from, the slot's
+// the one after the last.  Eight chunks' values are asked for at once, so the walk does not wait for memory at each.
+__global__ void __launch_bounds__(128)
+decay_carry_kernel(float* __restrict__ state, float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
+                   const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, int H, int D, int V) {
+    pdl_trigger();
+    pdl_wait();
+    const int seq = blockIdx.z, h = blockIdx.y, slot = seq_slot[seq];
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, d = e / V;
+    if (slot < 0 || e >= D * V) return;
+    size_t base = 0;
+    for (int s = 0; s < seq; ++s) base += (cu_seqlens[s + 1] - cu_seqlens[s] + DC_LEN - 1) / DC_LEN;
+    const int n = (cu_seqlens[seq + 1] - cu_seqlens[seq] + DC_LEN - 1) / DC_LEN;
+    float4* sp = reinterpret_cast<float4*>(state + ((size_t)slot * H + h) * D * V + e);
+    float* cp = chunk_state + (base * H + h) * (size_t)D * V + e;
+    const float* dp = chunk_decay + (base * H + h) * (size_t)D + d;
+    const size_t step = (size_t)H * D * V, dstep = (size_t)H * D;
+    float4 S = *sp;
+    for (int c = 0; c < n; c += 8) {
+        float4 add[8];
+        float w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + i < n) add[i] = *reinterpret_cast<const float4*>(cp + (c + i) * step), w[i] = dp[(c + i) * dstep];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + i < n) {
+                *reinterpret_cast<float4*>(cp + (c + i) * step) = S;
+                S = make_float4(fmaf(w[i], S.x, add[i].x), fmaf(w[i], S.y, add[i].y), fmaf(w[i], S.z, add[i].z), fmaf(w[i], S.w, add[i].w));
+            }
+    }
+    *sp = S;
+}
+
+template <int MODE, int DMAX>
+static int launch_decay_chunks(const bf16* qk, const bf16* v, const bf16* raw, float* out, float* state, float* chunk_state, float* chunk_decay,
+                               const DcArgs& a, int n_seqs, int max_chunks, cudaStream_t stream) {
+    const int VB = a.V < 128 ? a.V : 128;
+    const DcSmem add = dc_layout(a.D, VB, MODE == DC_SIGMOID, false), res = dc_layout(a.D, VB, MODE == DC_SIGMOID, true);
+    cudaError_t e = cudaFuncSetAttribute(decay_chunk_kernel<MODE, false, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)add.total);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(decay_chunk_kernel<MODE, true, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res.total);
+    if (e != cudaSuccess) return bfi_fail("decay_chunks: cannot reserve %zu bytes of shared memory: %s", res.total, cudaGetErrorString(e));
+    const dim3 grid(a.H * a.v_blocks, n_seqs, max_chunks);
+    bfi_launch(decay_chunk_kernel<MODE, false, DMAX>, grid, dim3(dc_warps(MODE, false) * 32), add.total, stream, qk, v, raw, out, chunk_state,
+               chunk_decay, a);
+    bfi_launch(decay_carry_kernel, dim3((a.D * a.V + 511) / 512, a.H, n_seqs), dim3(128), 0, stream, state, chunk_state, (const float*)chunk_decay,
+               a.cu_seqlens, a.seq_slot, a.H, a.D, a.V);
+    bfi_launch(decay_chunk_kernel<MODE, true, DMAX>, grid, dim3(dc_warps(MODE, true) * 32), res.total, stream, qk, v, raw, out, chunk_state,
+               chunk_decay, a);
+    return bfi_check_launch("decay_chunks");
+}
+
+// The arguments of bfi_decay_scan for bfloat16 inputs, with scratch for every chunk of 64 tokens.  Returns 2 ("not taken")
+// for sizes this kernel does not handle; the caller then runs the general one.
+extern "C" int bfi_decay_chunks_bf16(const void* qk, long qk_stride, int q_off, int k_off, const void* vsrc, long v_stride, int v_off,
+                                     const void* raw, long r_stride, int r_off, float* out, long out_stride, float* state,
+                                     const int* cu_seqlens, const int* seq_slot, int n_seqs, int H, int D, int V, int heads_per_group,
+                                     int mode, float q_scale, float inv_tau, const float* bias, const float* rate, const float* skip,
+                                     int max_chunks, float* chunk_state, float* chunk_decay, cudaStream_t stream) {
+    BFI_REQUIRE(H > 0 && D > 0 && V > 0, "decay_chunks: bad sizes heads=%d dim=%d vdim=%d", H, D, V);
+    BFI_REQUIRE(heads_per_group > 0 && H % heads_per_group == 0, "decay_chunks: %d heads do not form groups of %d", H, heads_per_group);
+    BFI_REQUIRE(mode == DC_STEP || mode == DC_SIGMOID, "decay_chunks: unknown decay form %d", mode);
+    BFI_REQUIRE(bias != nullptr && (mode != DC_STEP || rate != nullptr), "decay_chunks: the decay's constants are missing");
+    BFI_REQUIRE(out_stride >= (long)H * V, "decay_chunks: output stride shorter than the heads");
+    BFI_REQUIRE(max_chunks > 0 && chunk_state != nullptr && chunk_decay != nullptr, "decay_chunks: the chunks' count and scratch are missing");
+    if (n_seqs <= 0) return 0;
+    if (D % 16 != 0 || D > 128 || V % 16 != 0 || n_seqs > 65535 || max_chunks > 65535 || H > 65535) return 2;
+    // q, k, v and the decays per row are read in 16-byte pieces, the state is moved in 16-byte ones, outputs written in 8-byte ones
+    if (((uintptr_t)qk & 15) || ((uintptr_t)vsrc & 15) || qk_stride % 8 || v_stride % 8 || q_off % 8 || k_off % 8 || v_off % 8) return 2;
+    if (((uintptr_t)out & 7) || out_stride % 2 || ((uintptr_t)state & 15) || ((uintptr_t)chunk_state & 15)) return 2;
+    if (mode == DC_SIGMOID && (((uintptr_t)raw & 15) || r_stride % 8 || r_off % 8 || ((uintptr_t)bias & 15))) return 2;
+    DcArgs a;
+    a.qk_stride = qk_stride, a.v_stride = v_stride, a.r_stride = r_stride, a.out_stride = out_stride;
+    a.q_off = q_off, a.k_off = k_off, a.v_off = v_off, a.r_off = r_off;
+    a.H = H, a.D = D, a.V = V, a.heads_per_group = heads_per_group, a.v_blocks = (V + 127) / 128;
+    a.q_scale = q_scale, a.inv_tau = inv_tau, a.bias = bias, a.rate = rate, a.skip = skip;
+    a.cu_seqlens = cu_seqlens, a.seq_slot = seq_slot;
+#define BFI_DC(M, DM)                                                                                                              \
+    return launch_decay_chunks<M, DM>((const bf16*)qk, (const bf16*)vsrc, (const bf16*)raw, out, state, chunk_state, chunk_decay, a, \
+                                      n_seqs, max_chunks, stream)
+    if (mode == DC_STEP) {
+        if (D <= 64) BFI_DC(DC_STEP, 64);
+        BFI_DC(DC_STEP, 128);
+    }
+    if (D <= 64) BFI_DC(DC_SIGMOID, 64);
+    BFI_DC(DC_SIGMOID, 128);
+#undef BFI_DC
+}
+
+BFI_TRACE_EXPORT(decay_chunked)

@@ -66,20 +66,6 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr) {
     return d;
 }
 
-// Two values into their terms: h, m and l of both, packed.
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-    h = *reinterpret_cast<uint32_t*>(&t);
-    a -= __uint_as_float(h << 16);
-    b -= __uint_as_float(h & 0xffff0000u);
-    t = __floats2bfloat162_rn(a, b);
-    m = *reinterpret_cast<uint32_t*>(&t);
-    a -= __uint_as_float(m << 16);
-    b -= __uint_as_float(m & 0xffff0000u);
-    t = __floats2bfloat162_rn(a, b);
-    l = *reinterpret_cast<uint32_t*>(&t);
-}
-
 // One output by float32 multiply-adds, k rising: for results that are not finite.
 __device__ __noinline__ float dot_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
     float s = 0.0f;

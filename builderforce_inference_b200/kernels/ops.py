@@ -585,6 +585,9 @@ def gated_rows(out: torch.Tensor, src: torch.Tensor, g: torch.Tensor, accumulate
 DECAY_STEP, DECAY_SIGMOID = 1, 2
 
 
+DECAY_CHUNK_TOKENS = 64      # the tensor-core form's chunks
+
+
 def decay_scan(qk: torch.Tensor, q_off: int, k_off: int, v: torch.Tensor, v_off: int, raw: torch.Tensor, r_off: int,
                out: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int,
                n_heads: int, dim: int, vdim: int, heads_per_group: int, mode: int, bias: torch.Tensor,
@@ -601,7 +604,8 @@ def decay_scan(qk: torch.Tensor, q_off: int, k_off: int, v: torch.Tensor, v_off:
     ``chunk_len`` > 0 runs the chunked form (chunks of a sequence side by side, then a carry over the
     chunks, then the earlier tokens' part of every output): ``chunk_state`` float32 with
     ``heads * dim * vdim`` values and ``chunk_decay`` with ``heads * dim`` for every chunk of the step;
-    ``max_chunks`` is the most chunks one sequence has.  ``single_tokens``: every sequence of the
+    ``max_chunks`` is the most chunks one sequence has.  bfloat16 inputs in chunks of 64 run on the tensor
+    cores where the sizes allow.  ``single_tokens``: every sequence of the
     step brings exactly one token (the state is then streamed through once)."""
     _need_cuda(qk, v, raw, out, state, cu_seqlens, seq_slot, bias, rate, skip)
     for t, what in ((qk, "q and k"), (v, "values"), (raw, "decay input"), (out, "recurrence output")):
@@ -628,6 +632,13 @@ def decay_scan(qk: torch.Tensor, q_off: int, k_off: int, v: torch.Tensor, v_off:
         for t, per in ((chunk_state, n_heads * dim * vdim), (chunk_decay, n_heads * dim)):
             if t is None or t.dtype != torch.float32 or not t.is_contiguous() or t.numel() < n_chunks * per or not t.is_cuda:
                 raise KernelError(f"decay_scan: the chunked form needs float32 scratch for {n_chunks} chunks")
+        if chunk_len == DECAY_CHUNK_TOKENS and qk.dtype == torch.bfloat16 and library("fast").call_optional(
+                "bfi_decay_chunks_bf16", _ptr(qk), c_long(qk.stride(0)), c_int(q_off), c_int(k_off), _ptr(v), c_long(v.stride(0)),
+                c_int(v_off), _ptr(raw), c_long(raw.stride(0)), c_int(r_off), _ptr(out), c_long(out.stride(0)), _ptr(state),
+                _ptr(cu_seqlens), _ptr(seq_slot), c_int(n_seqs), c_int(n_heads), c_int(dim), c_int(vdim), c_int(heads_per_group),
+                c_int(mode), c_float(q_scale), c_float(inv_tau), _ptr(bias), _ptr(rate), _ptr(skip), c_int(max_chunks),
+                _ptr(chunk_state), _ptr(chunk_decay), _stream()):
+            return
     library("core").call("bfi_decay_scan", _ptr(qk), c_long(qk.stride(0)), c_int(q_off), c_int(k_off), _ptr(v),
                          c_long(v.stride(0)), c_int(v_off), _ptr(raw), c_long(raw.stride(0)), c_int(r_off),
                          c_int(dtype_code(qk.dtype)), _ptr(out), c_long(out.stride(0)), _ptr(state), _ptr(cu_seqlens),

@@ -53,23 +53,29 @@ from ..kernels.linear import EPI_ACCUMULATE, EPI_STORE, linear
 from .base import MIXERS, Mixer, ParamSpec, StateNeed
 
 
-CHUNK_TOKENS = 64            # chunk length of the chunked recurrence
-CHUNKED_MIN_TOKENS = 192     # a step whose longest piece is shorter walks its tokens in order
+CHUNK_TOKENS = ops.DECAY_CHUNK_TOKENS      # chunk length of the chunked recurrence
+CHUNKED_MIN_TOKENS = 192     # a step whose longest piece is shorter walks its tokens in order ...
+# ... unless the tensor-core kernels take its sizes: these win from 32 tokens on (60 tokens, 32 heads: 24 against 90 us; 8 x 33 tokens,
+# 16 heads: 35 against 57 us, with a decay per row 47 against 52) while their scratch, heads times chunks, stays in L2
+# (64 x 64 tokens, 32 heads, a decay per row: 935 against 740 us)
+TENSOR_MIN_TOKENS, TENSOR_MAX_HEAD_CHUNKS = 32, 1024
 
 
 def _as_f32(t: torch.Tensor) -> torch.Tensor:
     return t.float().contiguous()
 
 
-def _chunking(ctx, per_chunk: int, per_decay: int) -> dict:
+def _chunking(ctx, n_heads: int, dim: int, vdim: int) -> dict:
     """The chunked form's arguments for a step with long pieces (none for short steps and single
     tokens): its scratch comes from the step's workspace."""
-    if ctx.max_seq_tokens < CHUNKED_MIN_TOKENS:
-        return {}
     n_chunks = ctx.n_tokens // CHUNK_TOKENS + ctx.n_seqs
+    if ctx.max_seq_tokens < CHUNKED_MIN_TOKENS:
+        tensor = ctx.act_dtype == torch.bfloat16 and dim % 16 == 0 and dim <= 128 and vdim % 16 == 0
+        if not tensor or ctx.max_seq_tokens < TENSOR_MIN_TOKENS or n_chunks * n_heads > TENSOR_MAX_HEAD_CHUNKS:
+            return {}
     return {"chunk_len": CHUNK_TOKENS, "max_chunks": (ctx.max_seq_tokens + CHUNK_TOKENS - 1) // CHUNK_TOKENS,
-            "chunk_state": ctx.rows("rec.chunk_state", per_chunk, torch.float32, n_rows=n_chunks),
-            "chunk_decay": ctx.rows("rec.chunk_decay", per_decay, torch.float32, n_rows=n_chunks)}
+            "chunk_state": ctx.rows("rec.chunk_state", n_heads * dim * vdim, torch.float32, n_rows=n_chunks),
+            "chunk_decay": ctx.rows("rec.chunk_decay", n_heads * dim, torch.float32, n_rows=n_chunks)}
 
 
 @MIXERS.register("state_space")
@@ -139,7 +145,7 @@ class StateSpaceMixer(Mixer):
         ops.decay_scan(xbc, inner + gn, inner, xbc, 0, proj, 2 * inner + 2 * gn, y, state, ctx.cu_seqlens, ctx.seq_slot,
                        ctx.n_seqs, self.n_heads, self.state, self.vdim, self.n_heads // self.groups, ops.DECAY_STEP,
                        self.dt_bias, rate=self.rate, skip=self.skip, few_tokens=ctx.max_seq_tokens == 1, single_tokens=single,
-                       **_chunking(ctx, self.n_heads * self.state * self.vdim, self.n_heads * self.state))
+                       **_chunking(ctx, self.n_heads, self.state, self.vdim))
         g = ctx.rows("ssm.gated", inner)
         ops.gated_group_norm(y, proj[:, :inner], self.norm, self.eps, g, self.norm_groups, gate_first=True)
         linear(g, self.w_o, target, epilogue)
@@ -202,7 +208,7 @@ class GatedLinearAttention(Mixer):
                        self.n_heads, self.dim, self.vdim, 1, ops.DECAY_SIGMOID, self.a_bias, q_scale=self.dim ** -0.5,
                        inv_tau=1.0 / self.tau, few_tokens=ctx.max_seq_tokens == 1,
                        single_tokens=ctx.max_seq_tokens == 1 and ctx.n_tokens == ctx.n_seqs,
-                       **_chunking(ctx, self.n_heads * self.dim * self.vdim, self.n_heads * self.dim))
+                       **_chunking(ctx, self.n_heads, self.dim, self.vdim))
         y = ctx.rows("gla.y", vv)
         ops.gated_group_norm(o, proj[:, 2 * qk + vv:2 * qk + 2 * vv], self.norm, self.eps, y, self.n_heads, gate_first=False)
         linear(y, self.w_o, target, epilogue)

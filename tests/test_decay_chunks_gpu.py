@@ -1,0 +1,99 @@
+"""The recurrences with a decay per token on the tensor cores (chunks of 64 tokens) against a 64-bit walk in order, beside the
+float32 kernel that walks in order on the same data."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+F64 = torch.float64
+
+
+def data(mode, lens, H, G, D, V, seed, strong=False):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    n = sum(lens)
+    c = {"v": r(n, H * V).bfloat16(), "state": 0.3 * r(len(lens), H, D, V), "mode": mode}
+    if mode == "step":
+        c.update(qk=r(n, 2 * G * D).bfloat16(), raw=r(n, H).bfloat16(), hpg=H // G, bias=r(H) - 3.0, skip=r(H), q_scale=1.0,
+                 rate=torch.exp(r(H)) * (60.0 if strong else 1.0), inv_tau=1.0)
+    else:
+        c.update(qk=r(n, 2 * H * D).bfloat16(), raw=(2.0 * r(n, H * D)).bfloat16(), hpg=1, bias=(-9.0 if strong else 1.0) + r(H * D),
+                 skip=None, rate=None, q_scale=D ** -0.5, inv_tau=1.0 if strong else 0.125)
+    return c
+
+
+def in_order(c, lens, H, D, V):
+    qk, v, raw = c["qk"].to(F64), c["v"].to(F64), c["raw"].to(F64)
+    at, groups, outs, states = 0, H // c["hpg"], [], []
+    for i, n in enumerate(lens):
+        S = c["state"][i].to(F64)
+        for t in range(at, at + n):
+            q = qk[t, :groups * D].view(groups, D).repeat_interleave(c["hpg"], 0) * c["q_scale"]
+            k = qk[t, groups * D:].view(groups, D).repeat_interleave(c["hpg"], 0)
+            x = v[t].view(H, V)
+            if c["mode"] == "step":
+                step = torch.nn.functional.softplus(raw[t] + c["bias"].to(F64))
+                S = torch.exp(-c["rate"].to(F64) * step)[:, None, None] * S + k[:, :, None] * (step[:, None] * x)[:, None]
+            else:
+                a = torch.exp(torch.nn.functional.logsigmoid(raw[t] + c["bias"].to(F64)) * c["inv_tau"]).view(H, D)
+                S = a[:, :, None] * S + k[:, :, None] * x[:, None]
+            o = (q[:, None] @ S)[:, 0]
+            outs.append((o + (c["skip"].to(F64)[:, None] * x if c["skip"] is not None else 0.0)).reshape(-1))
+        at += n
+        states.append(S)
+    return torch.stack(outs), torch.stack(states)
+
+
+def run(c, lens, H, D, V, chunk_len):
+    from builderforce_inference_b200.kernels import ops
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    kw = {}
+    if chunk_len:
+        n_chunks = cu[-1] // chunk_len + len(lens)
+        kw = {"chunk_len": chunk_len, "max_chunks": (max(lens) + chunk_len - 1) // chunk_len,
+              "chunk_state": torch.full((n_chunks, H * D * V), float("nan"), device=DEV),
+              "chunk_decay": torch.full((n_chunks, H * D), float("nan"), device=DEV)}
+    out = torch.full((cu[-1], H * V), float("nan"), device=DEV)
+    state = c["state"].clone()
+    groups = H // c["hpg"]
+    ops.decay_scan(c["qk"], 0, groups * D, c["v"], 0, c["raw"], 0, out, state, torch.tensor(cu, dtype=torch.int32, device=DEV),
+                   torch.arange(len(lens), dtype=torch.int32, device=DEV), len(lens), H, D, V, c["hpg"],
+                   ops.DECAY_STEP if c["mode"] == "step" else ops.DECAY_SIGMOID, c["bias"], rate=c["rate"], skip=c["skip"],
+                   q_scale=c["q_scale"], inv_tau=c["inv_tau"], **kw)
+    return out, state
+
+
+def err(x, ref):
+    return float((x.to(F64) - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("mode", ["step", "sigmoid"])
+@pytest.mark.parametrize("lens,H,G,D,V", [([64], 2, 1, 16, 16), ([1, 65, 130], 4, 2, 64, 64), ([300, 63, 17], 4, 4, 128, 128),
+                                          ([200], 2, 2, 48, 112), ([129], 2, 1, 80, 144), ([700, 2], 6, 2, 128, 64)])
+def test_chunks_on_the_tensor_cores(mode, lens, H, G, D, V):
+    c = data(mode, lens, H, G, D, V, D + V + len(lens))
+    ref, S = in_order(c, lens, H, D, V)
+    plain, S_plain = run(c, lens, H, D, V, 0)
+    out, S_out = run(c, lens, H, D, V, 64)
+    # float32 throughout: a few roundings of every term, as in the walk in order
+    assert err(out, ref) < 6e-7 and err(S_out, S) < 6e-7
+    assert err(out, ref) < 1.3 * err(plain, ref) + 1e-7 and err(S_out, S) < 1.3 * err(S_plain, S) + 1e-7
+
+
+@pytest.mark.parametrize("mode", ["step", "sigmoid"])
+def test_decays_that_leave_nothing_and_values_that_are_not_finite(mode):
+    lens, H, G, D, V = [150, 64], 4, 2, 32, 48
+    c = data(mode, lens, H, G, D, V, 5, strong=True)          # a chunk's decays multiply to less than any float32
+    ref, S = in_order(c, lens, H, D, V)
+    out, S_out = run(c, lens, H, D, V, 64)
+    assert err(out, ref) < 6e-7 and err(S_out, S) < 6e-7
+    c = data(mode, lens, H, G, D, V, 6)
+    c["v"][100, 3] = float("inf")                             # token 100 of the first sequence, head 0, value 3
+    c["qk"][155, 1] = float("nan")                            # a query of the second sequence's token 5: that token alone
+    plain, S_plain = run(c, lens, H, D, V, 0)
+    out, S_out = run(c, lens, H, D, V, 64)
+    same = torch.isfinite(plain)
+    assert torch.equal(torch.isfinite(out), same) and torch.equal(torch.isfinite(S_out), torch.isfinite(S_plain))
+    assert bool(same[:100].all()) and err(out[same], plain[same].to(F64)) < 2e-6
