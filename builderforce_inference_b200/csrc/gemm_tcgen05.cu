@@ -473,12 +473,14 @@ __device__ __forceinline__ void tp_pre_store(float (&v)[16], int epilogue, const
     }
 }
 
-template <int HALVES, bool MAPPED>
+// GROUPED: `groups` products of one size in one launch, operands out of maps with the group as third coordinate, the
+// outputs `c_step` elements apart (the heads of an attention whose weights act head by head, say).
+template <int HALVES, bool MAPPED, bool GROUPED>
 __global__ void __launch_bounds__(TP_THREADS, 1)
 gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                            void* __restrict__ C, int c_dtype, long ldc, int M, int N, int K, int tiles_m, int tiles_n,
-                            int tile_n, int n_stages, int epilogue, GateAct gate, int vec_ok, int* __restrict__ status,
-                            TcWaits waits) {
+                            void* __restrict__ C0, int c_dtype, long ldc, int M, int N, int K, int tiles_m, int tiles_n,
+                            int tile_n, int n_stages, int epilogue, GateAct gate, int vec_ok, int groups, long c_step,
+                            int* __restrict__ status, TcWaits waits) {
     const uint32_t spin_limit = waits.spin_limit;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -493,7 +495,11 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kb = (K + TC_BK - 1) / TC_BK;
-    const int n_tiles = tiles_m * tiles_n;
+    const int group_tiles = tiles_m * tiles_n, n_tiles = group_tiles * (GROUPED ? groups : 1);
+    auto load = [](void* dst, const CUtensorMap* map, int x, int y, int group, uint64_t* bar) {
+        if (GROUPED) tma_load_3d(dst, map, x, y, group, bar);
+        else tma_load_2d(dst, map, x, y, bar);
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < n_stages; ++s) {
@@ -518,7 +524,9 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     pdl_trigger();                                 // the kernel after this one may start its own preamble
 
     // tiles in bands of 8 token tiles: blocks that run together share W tiles and A tiles in L2
-    auto tile_coords = [&](int tile, int& tm, int& tn) {
+    auto tile_coords = [&](int tile, int& tm, int& tn, int& tg) {
+        tg = 0;
+        if (GROUPED) tg = tile / group_tiles, tile -= tg * group_tiles;
         const int band = 8;
         const int per_band = band * tiles_n;
         const int b = tile / per_band, r = tile - b * per_band;
@@ -532,8 +540,8 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             int it = 0;                                            // k blocks issued so far, over all tiles
             bool first = true;
             for (int tile = blockIdx.x; tile < n_tiles && !s_flag[0] && !waits.hold_producer; tile += gridDim.x) {
-                int tm, tn;
-                tile_coords(tile, tm, tn);
+                int tm, tn, tg;
+                tile_coords(tile, tm, tn, tg);
                 int i0 = 0;
                 if (first) {
                     // W does not depend on the kernel before this one: the first stages' W halves travel
@@ -541,12 +549,11 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                     const int early = n_kb < n_stages ? n_kb : n_stages;
                     for (int i = 0; i < early; ++i) {
                         mbar_expect_tx(&full[i], stage_bytes);
-                        tma_load_2d(smem + (size_t)i * stage_bytes + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n,
-                                    &full[i]);
+                        load(smem + (size_t)i * stage_bytes + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[i]);
                     }
                     pdl_wait();
                     for (int i = 0; i < early; ++i)
-                        tma_load_2d(smem + (size_t)i * stage_bytes, &map_a, i * TC_BK, tm * TILE_TOKENS, &full[i]);
+                        load(smem + (size_t)i * stage_bytes, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[i]);
                     it = i0 = early;
                     first = false;
                 }
@@ -560,8 +567,8 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                     }
                     unsigned char* stage = smem + (size_t)s * stage_bytes;
                     mbar_expect_tx(&full[s], stage_bytes);
-                    tma_load_2d(stage, &map_a, i * TC_BK, tm * TILE_TOKENS, &full[s]);
-                    tma_load_2d(stage + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, &full[s]);
+                    load(stage, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[s]);
+                    load(stage + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[s]);
                 }
             }
             if (first) pdl_wait();
@@ -622,8 +629,9 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         const int quad = warp & 3;
         int local = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
-            int tm, tn;
-            tile_coords(tile, tm, tn);
+            int tm, tn, tg;
+            tile_coords(tile, tm, tn, tg);
+            void* const C = GROUPED ? static_cast<unsigned char*>(C0) + (size_t)tg * c_step * (c_dtype == BFI_F32 ? 4 : 2) : C0;
             const int full_idx = HALVES == 1 ? (local & 1) : 0;
             const uint32_t full_parity = HALVES == 1 ? (uint32_t)((local >> 1) & 1) : (uint32_t)(local & 1);
             if (epilogue == EPI_ACCUMULATE) {
@@ -804,8 +812,9 @@ struct MapKey {
     const void* ptr;
     long rows, cols, ld;
     int box_rows;
+    long groups, step;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows;
+        return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && groups == o.groups && step == o.step;
     }
 };
 struct MapKeyHash {
@@ -814,6 +823,8 @@ struct MapKeyHash {
         h = h * 1000003u ^ std::hash<long>()(k.rows);
         h = h * 1000003u ^ std::hash<long>()(k.cols);
         h = h * 1000003u ^ std::hash<long>()(k.ld);
+        h = h * 1000003u ^ std::hash<long>()(k.groups);
+        h = h * 1000003u ^ std::hash<long>()(k.step);
         return h * 1000003u ^ std::hash<int>()(k.box_rows);
     }
 };
@@ -821,7 +832,12 @@ static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 static std::mutex g_maps_mutex;
 
 int bfi_tensor_map_bf16(const void* ptr, long rows, long cols, long ld, int box_rows, CUtensorMap* out) {
-    MapKey key{ptr, rows, cols, ld, box_rows};
+    return bfi_tensor_map_groups_bf16(ptr, rows, cols, ld, 0, 0, box_rows, out);
+}
+
+// `groups` 0: a plain matrix (two coordinates).
+int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out) {
+    MapKey key{ptr, rows, cols, ld, box_rows, groups, step};
     std::lock_guard<std::mutex> lock(g_maps_mutex);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) {
@@ -830,12 +846,12 @@ int bfi_tensor_map_bf16(const void* ptr, long rows, long cols, long ld, int box_
     }
     EncodeTiledFn fn = encode_fn();
     if (!fn) return bfi_fail("gemm_tcgen05: the driver does not export cuTensorMapEncodeTiled");
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {TC_BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)groups};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)step * 2};
+    cuuint32_t box[3] = {TC_BK, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMap m;
-    CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+    CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups > 0 ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return bfi_fail("gemm_tcgen05: cuTensorMapEncodeTiled failed with code %d", (int)r);
@@ -945,14 +961,14 @@ static int launch_tc_prefill(const void* A, long lda, const void* W, long ldw, v
     static bool configured = false;
     const int n_sm = bfi_sm_count();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e != cudaSuccess)
             return bfi_fail("gemm_tcgen05: cannot reserve %zu bytes of shared memory: %s", (size_t)TP_SMEM, cudaGetErrorString(e));
         configured = true;
@@ -1000,10 +1016,10 @@ static int launch_tc_prefill(const void* A, long lda, const void* W, long ldw, v
     const int elem = dtype_size(c_dtype);
     const int vec_ok = ((ldc * elem) % 16 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
     const bool mapped = tc_mapped(epilogue);
-    auto kernel = halves == 2 ? (mapped ? gemm_tcgen05_prefill_kernel<2, true> : gemm_tcgen05_prefill_kernel<2, false>)
-                              : (mapped ? gemm_tcgen05_prefill_kernel<1, true> : gemm_tcgen05_prefill_kernel<1, false>);
+    auto kernel = halves == 2 ? (mapped ? gemm_tcgen05_prefill_kernel<2, true, false> : gemm_tcgen05_prefill_kernel<2, false, false>)
+                              : (mapped ? gemm_tcgen05_prefill_kernel<1, true, false> : gemm_tcgen05_prefill_kernel<1, false, false>);
     bfi_launch(kernel, dim3(grid), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C, c_dtype, ldc, M, N, K, tiles_m, tiles_n, tile_n,
-               n_stages, epilogue, g_bfi_gate, vec_ok, status, waits);
+               n_stages, epilogue, g_bfi_gate, vec_ok, 1, 0L, status, waits);
     return bfi_check_launch("gemm_tcgen05_prefill");
 }
 
@@ -1045,6 +1061,53 @@ static int gemm_tcgen05_launch(const void* A, long lda, const void* W, long ldw,
 extern "C" int bfi_gemm_tcgen05_bf16(const void* A, long lda, const void* W, long ldw, void* C, int c_dtype, long ldc,
                                      int M, int N, int K, int epilogue, int* status, cudaStream_t stream) {
     return gemm_tcgen05_launch(A, lda, W, ldw, C, c_dtype, ldc, M, N, K, epilogue, status, stream, tc_waits_default());
+}
+
+// `groups` products of one size in one launch: C_g[M,N] = A_g[M,K] * W_g[N,K]^T, group g's A `a_step`, W `w_step` and C
+// `c_step` elements behind the group before.  Any number of rows (a tile is 128 of them).  What bounds
+// it is its outputs (and, for few rows, its launch): 16 heads of an attention's latent space, 64 -> 512 and 512 -> 128 values,
+// over 2,048 tokens: 11 and 11 us where a launch per head took 157 each; over 64 tokens: 3.3 and 5.2 us where the
+// CUDA-core kernels of latent.cu take 14.7 and 29.2; over one token: 3.2 and 5.2 where they take 6.1 and 8.7.
+// Returns as bfi_gemm_tcgen05_bf16.
+extern "C" int bfi_gemm_groups_bf16(const void* A, long lda, long a_step, const void* W, long ldw, long w_step, void* C, int c_dtype,
+                                    long ldc, long c_step, int groups, int M, int N, int K, int* status, cudaStream_t stream) {
+    BFI_REQUIRE(dtype_ok(c_dtype), "gemm_groups: unknown output dtype code %d", c_dtype);
+    BFI_REQUIRE(M >= 0 && N > 0 && K > 0 && groups > 0, "gemm_groups: bad sizes M=%d N=%d K=%d groups=%d", M, N, K, groups);
+    BFI_REQUIRE(status != nullptr, "gemm_groups: a status word is required");
+    if (M == 0) return 0;
+    // TMA: 16-byte aligned bases and strides; strides that do not overlap backwards
+    if (K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 || a_step % 8 != 0 || w_step % 8 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return 2;
+    if (lda < K || ldw < K || a_step <= 0 || w_step <= 0) return 2;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+        if (e != cudaSuccess) return bfi_fail("gemm_groups: cannot reserve %zu bytes of shared memory: %s", (size_t)TP_SMEM, cudaGetErrorString(e));
+        configured = true;
+    }
+    // as launch_tc_prefill, for one half of 128 tokens; narrow tiles where the groups alone leave SMs idle
+    const int tiles_m = (M + TP_TOKENS - 1) / TP_TOKENS, n_sm = bfi_sm_count(), n_kb = (K + TC_BK - 1) / TC_BK;
+    int tile_n = 32;
+    double best = -1.0;
+    for (int tn = TP_FEATS; tn >= 32; tn -= 16) {
+        const long t = (long)tiles_m * ((N + tn - 1) / tn) * groups;
+        const double cost = (double)((t + n_sm - 1) / n_sm) * (n_kb * (0.351 + 0.00048 * tn) + 1.0 + 0.008 * tn);
+        if (best < 0.0 || cost < best) best = cost, tile_n = tn;
+    }
+    const int tiles_n = (N + tile_n - 1) / tile_n;
+    const long tiles = (long)tiles_m * tiles_n * groups;
+    if (tiles > 0x7fffffffL) return 2;
+    int n_stages = TP_RING_BYTES / ((TP_TOKENS + tile_n) * TC_BK * 2);
+    if (n_stages > TP_MAX_STAGES) n_stages = TP_MAX_STAGES;
+    CUtensorMap ma, mw;
+    int rc = bfi_tensor_map_groups_bf16(A, M, K, lda, groups, a_step, TP_TOKENS, &ma);
+    if (rc) return rc;
+    rc = bfi_tensor_map_groups_bf16(W, N, K, ldw, groups, w_step, tile_n, &mw);
+    if (rc) return rc;
+    const int elem = dtype_size(c_dtype);
+    const int vec_ok = ((ldc * elem) % 16 == 0 && (c_step * elem) % 16 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
+    bfi_launch(gemm_tcgen05_prefill_kernel<1, false, true>, dim3((unsigned)(tiles < n_sm ? tiles : n_sm)), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C,
+               c_dtype, ldc, M, N, K, tiles_m, tiles_n, tile_n, n_stages, EPI_STORE, g_bfi_gate, vec_ok, groups, c_step, status, tc_waits_default());
+    return bfi_check_launch("gemm_groups");
 }
 
 // For the tests of the time-out path: the same launch, but every bounded wait gives up after

@@ -55,6 +55,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols));
 }
@@ -134,3 +140,6 @@ __host__ __device__ constexpr uint32_t umma_idesc(int m, int n) {
 // box_rows x 64 elements with the 128-byte swizzle.  Maps are cached by their arguments.
 // Returns 0, or 1 after recording an error.
 int bfi_tensor_map_bf16(const void* ptr, long rows, long cols, long ld, int box_rows, CUtensorMap* out);
+// The same for `groups` such matrices, each `step` elements behind the one before: x, row, group.  What lies past a
+// group's columns or rows reads as zero, whatever the memory there holds.
+int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out);

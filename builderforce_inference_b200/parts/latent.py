@@ -23,8 +23,8 @@ Launches: one product for queries, gate logits and down projection together; ``l
 tensor-core kernel over stacked (token, head) rows, cut into key ranges when a step has few rows;
 otherwise the general paged kernel, and the gate then waits for ``latent_expand``);
 ``latent_expand`` (``W_uv`` and the gate); the output product, which adds into the residual stream.
-In bfloat16 steps of more than ``PRODUCT_MIN_TOKENS`` tokens, ``latent_absorb`` and ``latent_expand``
-are one tensor-core product per head each, on slices of the same buffers.
+In bfloat16 (when every slice starts on 16 bytes) ``latent_absorb`` and ``latent_expand`` are tensor-core
+products of all heads in one launch each, on slices of the same buffers; they are faster from one token on.
 
 Further variants, each a parameter.  ``q_rank``: the queries go through a latent of their own,
 ``q = W_uq norm(W_dq h)`` (an RMS norm with a weight of ``q_rank`` values); the first product then
@@ -51,7 +51,6 @@ from .base import MIXERS, POSITION_ENCODINGS, KVNeed, Mixer, ParamSpec, PartSpec
 @MIXERS.register("latent_attention")
 class LatentAttention(Mixer):
     graph_safe = True
-    PRODUCT_MIN_TOKENS = 64     # steps of more tokens: W_uk^T and W_uv as one matrix product per head
 
     def __init__(self, width: int, n_heads: int, dim: int, rot_dim: int, v_dim: int, kv_rank: int,
                  position: Optional[PartSpec] = None, eps: float = 1e-6, scale: Optional[float] = None,
@@ -165,7 +164,7 @@ class LatentAttention(Mixer):
         self.w_in = torch.cat(parts, dim=0).contiguous() if len(parts) > 1 else parts[0]
         self.w_uk = tensors["uk_proj"].contiguous()
         self.w_uv = tensors["uv_proj"].contiguous()
-        # steps of many tokens take W_uk^T and W_uv to the tensor cores head by head: W_uk_a^T as a
+        # W_uk^T and W_uv go to the tensor cores head by head: W_uk_a^T as a
         # matrix of its own ([kv_rank, dim]), when every slice starts on 16 bytes
         sizes = (self.dim, self.dim + self.rot_dim, self.kv_rank, self.kv_rank + self.rot_dim, self.v_dim, self.n_cols)
         self.w_uk_t = None
@@ -202,11 +201,10 @@ class LatentAttention(Mixer):
         qa = ctx.rows("latent.q", a * (r + rd))
         ops.latent_prepare(proj, qa, a, self.dim, rd, r, self.kv_off, self.dkv_norm, self.eps, table, rot_used,
                            ctx.token_pos, ctx.token_slot, kv, run.writes_cache, ctx.status)
-        products = self.w_uk_t is not None and proj.dtype == torch.bfloat16 and ctx.n_tokens > self.PRODUCT_MIN_TOKENS
+        products = self.w_uk_t is not None and proj.dtype == torch.bfloat16
         if products:
             dq = self.dim + rd
-            for i in range(a):
-                linear(proj[:, i * dq:i * dq + self.dim], self.w_uk_t[i], qa[:, i * (r + rd):i * (r + rd) + r], EPI_STORE)
+            self._head_products(proj[:, :self.dim], dq, self.w_uk_t, qa[:, :r], r + rd)
         else:
             ops.latent_absorb(proj, self.w_uk, qa, ctx.token_slot, a, self.dim, rd, r)
         lat = ctx.rows("latent.out", a * r)
@@ -217,13 +215,19 @@ class LatentAttention(Mixer):
         out = ctx.rows("attn.out", a * self.v_dim)
         if products and (gate is None or self.gate_values):
             dv = self.v_dim
-            for i in range(a):
-                linear(lat[:, i * r:(i + 1) * r], self.w_uv[i * dv:(i + 1) * dv], out[:, i * dv:(i + 1) * dv], EPI_STORE)
+            self._head_products(lat[:, :r], r, self.w_uv.view(a, dv, r), out[:, :dv], dv)
             if gate is not None:
                 ops.sigmoid_gate(out, gate, 1)
         else:
             ops.latent_expand(lat, self.w_uv, gate, out, ctx.token_slot, a, self.v_dim, r)
         linear(out, self.w_o, target, epilogue)
+
+    @staticmethod
+    def _head_products(x, x_step: int, w, out, out_step: int) -> None:
+        """``out_a = x_a @ w_a.T`` for every head; ``x`` and ``out`` are the first head's columns."""
+        from ..kernels import fast_ops
+        if not fast_ops.gemm_groups(x, x_step, w, out, out_step):
+            raise RuntimeError("latent attention: the heads' products were refused")     # w_uk_t exists where every slice is aligned
 
     def attend(self, ctx, qa, lat, kv, gate=None) -> bool:
         """The attention in the latent space; True if it has multiplied the heads' outputs by their
