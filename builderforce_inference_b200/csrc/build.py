@@ -28,7 +28,8 @@ LIBRARIES: Dict[str, List[str]] = {
              "recurrence.cu", "channelwise.cu", "mlstm.cu", "streams.cu", "moe.cu", "latent.cu", "sublayer_out.cu", "sampling.cu", "utility.cu"],
     "fast": ["errors.cu", "skinny_gemm.cu", "attention_decode.cu", "attention_prefill.cu", "gemm_tcgen05.cu",
              "attention_prefill_tcgen05.cu", "attention_latent.cu", "weight_stream.cu", "lightning_chunked.cu",
-             "mlstm_chunked.cu", "decay_chunked.cu"],
+             "mlstm_chunked.cu", "decay_chunked.cu",
+             "moe_sorted.cu"],
 }
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -473,14 +473,20 @@ __device__ __forceinline__ void tp_pre_store(float (&v)[16], int epilogue, const
     }
 }
 
-// GROUPED: `groups` products of one size in one launch, operands out of maps with the group as third coordinate, the
+// KIND TP_GROUPS: `groups` products of one size in one launch, operands out of maps with the group as third coordinate, the
 // outputs `c_step` elements apart (the heads of an attention whose weights act head by head, say).
-template <int HALVES, bool MAPPED, bool GROUPED>
+// KIND TP_TILES: every tile of 128 rows has a W of its own, the third coordinate of W's map: `tile_group` names it, and
+// `*tiles_used` says how many such tiles there are (both left by an earlier kernel, so nothing of a tile is asked for before it
+// is done).
+#define TP_PLAIN 0
+#define TP_GROUPS 1
+#define TP_TILES 2
+template <int HALVES, bool MAPPED, int KIND>
 __global__ void __launch_bounds__(TP_THREADS, 1)
 gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                             void* __restrict__ C0, int c_dtype, long ldc, int M, int N, int K, int tiles_m, int tiles_n,
                             int tile_n, int n_stages, int epilogue, GateAct gate, int vec_ok, int groups, long c_step,
-                            int* __restrict__ status, TcWaits waits) {
+                            const int* __restrict__ tile_group, const int* __restrict__ tiles_used, int* __restrict__ status, TcWaits waits) {
     const uint32_t spin_limit = waits.spin_limit;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -495,9 +501,13 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kb = (K + TC_BK - 1) / TC_BK;
-    const int group_tiles = tiles_m * tiles_n, n_tiles = group_tiles * (GROUPED ? groups : 1);
-    auto load = [](void* dst, const CUtensorMap* map, int x, int y, int group, uint64_t* bar) {
-        if (GROUPED) tma_load_3d(dst, map, x, y, group, bar);
+    const int group_tiles = tiles_m * tiles_n;
+    auto load_a = [](void* dst, const CUtensorMap* map, int x, int y, int group, uint64_t* bar) {
+        if (KIND == TP_GROUPS) tma_load_3d(dst, map, x, y, group, bar);
+        else tma_load_2d(dst, map, x, y, bar);
+    };
+    auto load_w = [](void* dst, const CUtensorMap* map, int x, int y, int group, uint64_t* bar) {
+        if (KIND != TP_PLAIN) tma_load_3d(dst, map, x, y, group, bar);
         else tma_load_2d(dst, map, x, y, bar);
     };
 
@@ -522,17 +532,23 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_trigger();                                 // the kernel after this one may start its own preamble
+    if (KIND == TP_TILES) {
+        pdl_wait();
+        tiles_m = min(tiles_m, *tiles_used);
+    }
+    const int n_tiles = KIND == TP_TILES ? tiles_m * tiles_n : group_tiles * (KIND == TP_GROUPS ? groups : 1);
 
     // tiles in bands of 8 token tiles: blocks that run together share W tiles and A tiles in L2
     auto tile_coords = [&](int tile, int& tm, int& tn, int& tg) {
         tg = 0;
-        if (GROUPED) tg = tile / group_tiles, tile -= tg * group_tiles;
+        if (KIND == TP_GROUPS) tg = tile / group_tiles, tile -= tg * group_tiles;
         const int band = 8;
         const int per_band = band * tiles_n;
         const int b = tile / per_band, r = tile - b * per_band;
         const int rows_here = min(band, tiles_m - b * band);
         tn = r / rows_here;
         tm = b * band + (r - tn * rows_here);
+        if (KIND == TP_TILES) tg = tile_group[tm];
     };
 
     if (warp == 0) {
@@ -549,11 +565,11 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                     const int early = n_kb < n_stages ? n_kb : n_stages;
                     for (int i = 0; i < early; ++i) {
                         mbar_expect_tx(&full[i], stage_bytes);
-                        load(smem + (size_t)i * stage_bytes + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[i]);
+                        load_w(smem + (size_t)i * stage_bytes + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[i]);
                     }
                     pdl_wait();
                     for (int i = 0; i < early; ++i)
-                        load(smem + (size_t)i * stage_bytes, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[i]);
+                        load_a(smem + (size_t)i * stage_bytes, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[i]);
                     it = i0 = early;
                     first = false;
                 }
@@ -567,8 +583,8 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
                     }
                     unsigned char* stage = smem + (size_t)s * stage_bytes;
                     mbar_expect_tx(&full[s], stage_bytes);
-                    load(stage, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[s]);
-                    load(stage + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[s]);
+                    load_a(stage, &map_a, i * TC_BK, tm * TILE_TOKENS, tg, &full[s]);
+                    load_w(stage + TILE_TOKENS * TC_BK * 2, &map_w, i * TC_BK, tn * tile_n, tg, &full[s]);
                 }
             }
             if (first) pdl_wait();
@@ -631,7 +647,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
             int tm, tn, tg;
             tile_coords(tile, tm, tn, tg);
-            void* const C = GROUPED ? static_cast<unsigned char*>(C0) + (size_t)tg * c_step * (c_dtype == BFI_F32 ? 4 : 2) : C0;
+            void* const C = KIND == TP_GROUPS ? static_cast<unsigned char*>(C0) + (size_t)tg * c_step * (c_dtype == BFI_F32 ? 4 : 2) : C0;
             const int full_idx = HALVES == 1 ? (local & 1) : 0;
             const uint32_t full_parity = HALVES == 1 ? (uint32_t)((local >> 1) & 1) : (uint32_t)(local & 1);
             if (epilogue == EPI_ACCUMULATE) {
@@ -961,14 +977,14 @@ static int launch_tc_prefill(const void* A, long lda, const void* W, long ldw, v
     static bool configured = false;
     const int n_sm = bfi_sm_count();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, TP_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, false, TP_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, true, TP_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+            e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<2, true, TP_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e != cudaSuccess)
             return bfi_fail("gemm_tcgen05: cannot reserve %zu bytes of shared memory: %s", (size_t)TP_SMEM, cudaGetErrorString(e));
         configured = true;
@@ -1016,10 +1032,10 @@ static int launch_tc_prefill(const void* A, long lda, const void* W, long ldw, v
     const int elem = dtype_size(c_dtype);
     const int vec_ok = ((ldc * elem) % 16 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
     const bool mapped = tc_mapped(epilogue);
-    auto kernel = halves == 2 ? (mapped ? gemm_tcgen05_prefill_kernel<2, true, false> : gemm_tcgen05_prefill_kernel<2, false, false>)
-                              : (mapped ? gemm_tcgen05_prefill_kernel<1, true, false> : gemm_tcgen05_prefill_kernel<1, false, false>);
+    auto kernel = halves == 2 ? (mapped ? gemm_tcgen05_prefill_kernel<2, true, TP_PLAIN> : gemm_tcgen05_prefill_kernel<2, false, TP_PLAIN>)
+                              : (mapped ? gemm_tcgen05_prefill_kernel<1, true, TP_PLAIN> : gemm_tcgen05_prefill_kernel<1, false, TP_PLAIN>);
     bfi_launch(kernel, dim3(grid), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C, c_dtype, ldc, M, N, K, tiles_m, tiles_n, tile_n,
-               n_stages, epilogue, g_bfi_gate, vec_ok, 1, 0L, status, waits);
+               n_stages, epilogue, g_bfi_gate, vec_ok, 1, 0L, (const int*)nullptr, (const int*)nullptr, status, waits);
     return bfi_check_launch("gemm_tcgen05_prefill");
 }
 
@@ -1080,7 +1096,7 @@ extern "C" int bfi_gemm_groups_bf16(const void* A, long lda, long a_step, const 
     if (lda < K || ldw < K || a_step <= 0 || w_step <= 0) return 2;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<1, false, TP_GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
         if (e != cudaSuccess) return bfi_fail("gemm_groups: cannot reserve %zu bytes of shared memory: %s", (size_t)TP_SMEM, cudaGetErrorString(e));
         configured = true;
     }
@@ -1105,9 +1121,57 @@ extern "C" int bfi_gemm_groups_bf16(const void* A, long lda, long a_step, const 
     if (rc) return rc;
     const int elem = dtype_size(c_dtype);
     const int vec_ok = ((ldc * elem) % 16 == 0 && (c_step * elem) % 16 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
-    bfi_launch(gemm_tcgen05_prefill_kernel<1, false, true>, dim3((unsigned)(tiles < n_sm ? tiles : n_sm)), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C,
-               c_dtype, ldc, M, N, K, tiles_m, tiles_n, tile_n, n_stages, EPI_STORE, g_bfi_gate, vec_ok, groups, c_step, status, tc_waits_default());
+    bfi_launch(gemm_tcgen05_prefill_kernel<1, false, TP_GROUPS>, dim3((unsigned)(tiles < n_sm ? tiles : n_sm)), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C,
+               c_dtype, ldc, M, N, K, tiles_m, tiles_n, tile_n, n_stages, EPI_STORE, g_bfi_gate, vec_ok, groups, c_step,
+               (const int*)nullptr, (const int*)nullptr, status, tc_waits_default());
     return bfi_check_launch("gemm_groups");
+}
+
+// Rows in tiles of 128, every tile with a W of its own: C[m,N] = A[m,K] * W_g[N,K]^T with g = tile_group[m / 128], for the
+// first *tiles_used tiles of at most `tiles` (device memory, left by an earlier kernel of the stream: a routed
+// feed-forward's rows sorted by expert).  W_g is `w_step` elements behind the one before, `groups` of them; the epilogues are
+// bfi_gemm_tcgen05_bf16's but the adding one.  Returns as that.
+extern "C" int bfi_gemm_tiles_bf16(const void* A, long lda, const void* W, long ldw, long w_step, int groups, const int* tile_group,
+                                   const int* tiles_used, void* C, int c_dtype, long ldc, int tiles, int N, int K, int epilogue, int* status,
+                                   cudaStream_t stream) {
+    BFI_REQUIRE(dtype_ok(c_dtype), "gemm_tiles: unknown output dtype code %d", c_dtype);
+    BFI_REQUIRE(tiles >= 0 && N > 0 && K > 0 && groups > 0, "gemm_tiles: bad sizes tiles=%d N=%d K=%d groups=%d", tiles, N, K, groups);
+    BFI_REQUIRE(status != nullptr && tile_group != nullptr && tiles_used != nullptr, "gemm_tiles: the tiles' groups, their number and a status word are required");
+    BFI_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_SWIGLU || epilogue == BFI_EPI_RELU_SQUARED, "gemm_tiles: epilogue %d is not taken", epilogue);
+    if (epilogue == EPI_SWIGLU) BFI_REQUIRE(N % 2 == 0, "gemm_tiles: the gated epilogue needs an even N, got %d", N);
+    if (tiles == 0) return 0;
+    if (K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 || w_step % 8 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return 2;
+    if (lda < K || w_step <= 0 || tiles > (1 << 23)) return 2;
+    auto kernel = gemm_tcgen05_prefill_kernel<1, true, TP_TILES>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM);
+        if (e != cudaSuccess) return bfi_fail("gemm_tiles: cannot reserve %zu bytes of shared memory: %s", (size_t)TP_SMEM, cudaGetErrorString(e));
+        configured = true;
+    }
+    // the width with the least time by launch_tc_prefill's estimate, for the most tiles there can be
+    const int n_sm = bfi_sm_count(), n_kb = (K + TC_BK - 1) / TC_BK, M = tiles * TP_TOKENS;
+    int tile_n = TP_FEATS;
+    double best = -1.0;
+    for (int tn = TP_FEATS; tn >= 128; tn -= 16) {
+        const long t = (long)tiles * ((N + tn - 1) / tn);
+        const double cost = (double)((t + n_sm - 1) / n_sm) * (n_kb * (0.351 + 0.00048 * tn) + 2.0);
+        if (best < 0.0 || cost < best) best = cost, tile_n = tn;
+    }
+    const int tiles_n = (N + tile_n - 1) / tile_n;
+    const long all = (long)tiles * tiles_n;
+    if (all > 0x7fffffffL) return 2;
+    int n_stages = TP_RING_BYTES / ((TP_TOKENS + tile_n) * TC_BK * 2);
+    if (n_stages > TP_MAX_STAGES) n_stages = TP_MAX_STAGES;
+    CUtensorMap ma, mw;
+    int rc = bfi_tensor_map_bf16(A, M, K, lda, TP_TOKENS, &ma);
+    if (rc) return rc;
+    rc = bfi_tensor_map_groups_bf16(W, N, K, ldw, groups, w_step, tile_n, &mw);
+    if (rc) return rc;
+    const int vec_ok = ((ldc * dtype_size(c_dtype)) % 16 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
+    bfi_launch(kernel, dim3((unsigned)(all < n_sm ? all : n_sm)), dim3(TP_THREADS), TP_SMEM, stream, ma, mw, C, c_dtype, ldc, M, N, K, tiles, tiles_n,
+               tile_n, n_stages, epilogue, g_bfi_gate, vec_ok, groups, 0L, tile_group, tiles_used, status, tc_waits_default());
+    return bfi_check_launch("gemm_tiles");
 }
 
 // For the tests of the time-out path: the same launch, but every bounded wait gives up after

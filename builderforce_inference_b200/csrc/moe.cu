@@ -26,7 +26,8 @@
 // The experts' weights are two matrices for all experts, the layouts the dense products take as well:
 // W_gu [E * 2 * ff, width], expert e's gate row j at row 2 (e ff + j) and its up row right after it;
 // W_down [width, E * ff], expert e's columns at e ff .. (e + 1) ff.
-// When most experts are used anyway (many tokens), the dense products compute every expert for every
+// Longer prompts sort their pairs by expert instead (moe_sorted.cu).
+// When most experts are used anyway (up to 127 tokens, or most experts chosen by a token), the dense products compute every expert for every
 // token on the tensor cores and bfi_moe_weigh_dense multiplies the activations by the chosen experts'
 // weights (0 for the others) between the two products:  act[t, e ff + j] *= weight of e for token t.
 // An expert that every token uses may stand behind the routed ones in both matrices (`tail` more
@@ -257,6 +258,74 @@ moe_router_kernel(const T* __restrict__ h, long h_stride, const float* __restric
                         weight_scale, extra, lane, score_mode, group_top, dense_weight);
 }
 
+// The same for steps of many tokens: a block takes MR_TOKENS tokens, a warp two logits of half of them, so that a router row
+// is read once for four tokens and an input once for two rows, where a block per token reads all rows from L2 for itself
+// (2,048 tokens of 2,048 values, 16 experts and a gate: 54 -> 39 us with its launch).  Every logit is the same sums in the same order.
+#define MR_TOKENS 8
+#define MR_MANY 512          // from this many tokens on there is such a block for nearly every other SM
+template <typename T>
+__global__ void __launch_bounds__(512)
+moe_router_many_kernel(const T* __restrict__ h, long h_stride, const float* __restrict__ w_router,
+                       const float* __restrict__ correction, const int* __restrict__ token_slot, int* __restrict__ idx,
+                       float* __restrict__ weight, float* __restrict__ gate, int n_tokens, int width, int E, int top, int n_groups, int keep,
+                       float weight_scale, int extra, int score_mode, int group_top, float* __restrict__ dense_weight) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float sm[];
+    const int ld = width + 4, per = 2 * E + n_groups;
+    float* hs = sm;                                // [MR_TOKENS][width + 4]: rows of a multiple of 16 bytes
+    float* z = hs + MR_TOKENS * ld;                // [MR_TOKENS][E + 1]
+    float* scratch = z + MR_TOKENS * (E + 1);      // [MR_TOKENS][2 E + n_groups]
+    const int t0 = blockIdx.x * MR_TOKENS, n = min(MR_TOKENS, n_tokens - t0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    pdl_wait();
+    for (int t = 0; t < MR_TOKENS; ++t)
+        for (int j = threadIdx.x * 4; j < width; j += blockDim.x * 4) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t < n) {
+                const T* p = h + (size_t)(t0 + t) * h_stride + j;
+                x = make_float4(to_f32(p[0]), to_f32(p[1]), to_f32(p[2]), to_f32(p[3]));
+            }
+            *reinterpret_cast<float4*>(hs + t * ld + j) = x;
+        }
+    __syncthreads();
+    const int rows = E + (extra ? 1 : 0), pairs = (rows + 1) / 2;
+    for (int job = warp; job < 2 * pairs; job += n_warps) {
+        const int e0 = (job % pairs) * 2, e1 = min(e0 + 1, rows - 1), tb = job / pairs * 4;
+        const float *w0 = w_router + (size_t)e0 * width, *w1 = w_router + (size_t)e1 * width;
+        float a[2][4][2] = {};
+#pragma unroll 4
+        for (int j = lane * 4; j < width; j += 128) {
+            const float4 x0 = __ldg(reinterpret_cast<const float4*>(w0 + j)), x1 = __ldg(reinterpret_cast<const float4*>(w1 + j));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 b = *reinterpret_cast<const float4*>(hs + (tb + i) * ld + j);
+                a[0][i][0] = fmaf(x0.x, b.x, a[0][i][0]), a[0][i][1] = fmaf(x0.y, b.y, a[0][i][1]);
+                a[0][i][0] = fmaf(x0.z, b.z, a[0][i][0]), a[0][i][1] = fmaf(x0.w, b.w, a[0][i][1]);
+                a[1][i][0] = fmaf(x1.x, b.x, a[1][i][0]), a[1][i][1] = fmaf(x1.y, b.y, a[1][i][1]);
+                a[1][i][0] = fmaf(x1.z, b.z, a[1][i][0]), a[1][i][1] = fmaf(x1.w, b.w, a[1][i][1]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float d = warp_sum(a[r][i][0] + a[r][i][1]);
+                if (lane == 0 && (r == 0 || e1 > e0)) z[(tb + i) * (E + 1) + e0 + r] = d;
+            }
+    }
+    __syncthreads();
+    for (int t = warp; t < n; t += n_warps) {
+        if (token_slot[t0 + t] < 0) {              // padding row
+            if (dense_weight != nullptr)
+                for (int e = lane; e < E; e += 32) dense_weight[(size_t)(t0 + t) * E + e] = 0.0f;
+            continue;
+        }
+        float* s = scratch + (size_t)t * per;
+        moe_route_token(z + t * (E + 1), correction, idx, weight, gate, s, s + E, s + 2 * E, t0 + t, E, top, n_groups, keep, weight_scale, extra,
+                        lane, score_mode, group_top, dense_weight);
+    }
+}
+
 extern "C" int bfi_moe_router(const void* h, long h_stride, int dtype, const float* w_router, const float* correction,
                               const int* token_slot, int* idx, float* weight, float* gate, int n_tokens, int width, int E,
                               int top, int n_groups, int keep, float weight_scale, int extra, int score_mode, int group_top,
@@ -272,6 +341,23 @@ extern "C" int bfi_moe_router(const void* h, long h_stride, int dtype, const flo
     const size_t smem = (size_t)(width + 3 * E + 1 + n_groups) * sizeof(float);
     BFI_REQUIRE(smem <= 160 * 1024, "moe_router: width %d and %d experts do not fit shared memory", width, E);
     cudaError_t e = cudaSuccess;
+    const size_t many = ((size_t)MR_TOKENS * (width + 4 + 3 * E + 1 + n_groups)) * sizeof(float);
+    if (n_tokens >= MR_MANY && width % 4 == 0 && ((uintptr_t)w_router & 15) == 0 && many <= 110 * 1024) {
+        const int pairs = (E + (extra ? 1 : 0) + 1) / 2, warps = pairs < 16 ? pairs : 16;
+        const dim3 grid((n_tokens + MR_TOKENS - 1) / MR_TOKENS), block(32 * warps);
+#define BFI_MR(T)                                                                                                                             \
+    do {                                                                                                                                      \
+        e = cudaFuncSetAttribute(moe_router_many_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many);                           \
+        if (e == cudaSuccess)                                                                                                                  \
+            bfi_launch(moe_router_many_kernel<T>, grid, block, many, stream, (const T*)h, h_stride, w_router, correction, token_slot, idx, weight, \
+                       gate, n_tokens, width, E, top, n_groups, keep, weight_scale, extra, score_mode, group_top, dense_weight);                \
+    } while (0)
+        if (dtype == BFI_F32) BFI_MR(float);
+        else BFI_MR(bf16);
+#undef BFI_MR
+        if (e != cudaSuccess) return bfi_fail("moe_router: cannot reserve %zu bytes of shared memory: %s", many, cudaGetErrorString(e));
+        return bfi_check_launch("moe_router");
+    }
     if (dtype == BFI_F32) {
         if (smem > 48 * 1024) e = cudaFuncSetAttribute(moe_router_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)

@@ -385,3 +385,75 @@ def mlstm_chunks_bf16(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, ga
         c_long(gates.stride(0)), _ptr(bias_i), _ptr(bias_f), c_float(cap), c_float(q_scale), _ptr(out), c_long(out.stride(0)),
         _ptr(state), _ptr(tails), _ptr(cu_seqlens), _ptr(seq_slot), c_int(n_seqs), c_int(n_heads), c_int(dim), c_int(vdim),
         c_int(columns), _stream())
+
+
+MOE_TILE_ROWS = 128      # rows of a tile of ``gemm_tiles``: an expert's pairs begin on a multiple of it
+
+
+def moe_tiles(n_pairs: int, n_experts: int) -> int:
+    """The most tiles the pairs can fill: every expert may leave one partly filled."""
+    return min(n_pairs // MOE_TILE_ROWS + n_experts, n_pairs)
+
+
+def moe_sort(idx: torch.Tensor, token_slot: torch.Tensor, n_experts: int, pair_row: torch.Tensor, row_pair: torch.Tensor,
+             tile_expert: torch.Tensor, tiles_used: torch.Tensor) -> None:
+    """The (token, expert) pairs of ``idx`` (int32 ``[tokens, top]``) in rows sorted by expert: ``pair_row`` ``[tokens, top]``,
+    ``row_pair`` ``[tiles * 128]`` (-1: a row that fills a tile up), ``tile_expert`` ``[tiles]`` and ``tiles_used`` ``[1]``, all int32,
+    with ``tiles`` at least ``moe_tiles``.  Tokens with slot -1 have no pairs."""
+    n, top = idx.shape
+    tiles = moe_tiles(n * top, n_experts)
+    for t, least, what in ((idx, n * top, "idx"), (token_slot, n, "token slots"), (pair_row, n * top, "pair_row"),
+                           (row_pair, tiles * MOE_TILE_ROWS, "row_pair"), (tile_expert, tiles, "tile_expert"), (tiles_used, 1, "tiles_used")):
+        if t.dtype != torch.int32 or not t.is_contiguous() or t.numel() < least or not t.is_cuda:
+            raise KernelError(f"moe_sort: {what} must be contiguous int32 with at least {least} values")
+    library("fast").call("bfi_moe_sort", _ptr(idx), _ptr(token_slot), c_int(n), c_int(top), c_int(n_experts), _ptr(pair_row), _ptr(row_pair),
+                         _ptr(tile_expert), _ptr(tiles_used), _stream())
+
+
+def moe_gather(h: torch.Tensor, row_pair: torch.Tensor, tiles_used: torch.Tensor, top: int, out: torch.Tensor, weight=None, row_weight=None) -> None:
+    """``out[r] = h[token of row r]`` (zeros for filler) for the rows ``moe_sort`` made; with ``row_weight`` also its pair's ``weight``."""
+    _rows_2d(h, "feed-forward input")
+    width = h.shape[1]
+    if h.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or not out.is_contiguous() or out.shape[1] != width or out.shape[0] % MOE_TILE_ROWS != 0:
+        raise KernelError("moe_gather: bfloat16 rows of the input's width, whole tiles of them")
+    if row_pair.dtype != torch.int32 or row_pair.numel() < out.shape[0]:
+        raise KernelError("moe_gather: a pair per row")
+    for t, least in ((weight, h.shape[0] * top), (row_weight, out.shape[0])):
+        if t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or t.numel() < least):
+            raise KernelError("moe_gather: weights are contiguous float32")
+    library("fast").call("bfi_moe_gather", _ptr(h), c_long(h.stride(0)), _ptr(row_pair), _ptr(tiles_used), _ptr(weight), c_int(top), c_int(width),
+                         c_int(out.shape[0] // MOE_TILE_ROWS), _ptr(out), _ptr(row_weight), _stream())
+
+
+def gemm_tiles(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, tiles_used: torch.Tensor, out: torch.Tensor, epilogue: int) -> bool:
+    """``out[m] = a[m] @ w[tile_group[m // 128]].T`` for the rows of the first ``tiles_used`` tiles; ``w`` ``[groups, n, k]``."""
+    groups, n, k = w.shape
+    _rows_2d(a, "A")
+    _rows_2d(out, "C")
+    tiles = a.shape[0] // MOE_TILE_ROWS
+    cols = n // 2 if epilogue == 2 else n
+    if a.shape != (tiles * MOE_TILE_ROWS, k) or out.shape != (tiles * MOE_TILE_ROWS, cols) or w.stride(2) != 1 or a.dtype != torch.bfloat16 \
+            or w.dtype != torch.bfloat16 or tile_group.dtype != torch.int32 or tile_group.numel() < tiles:
+        raise KernelError(f"gemm_tiles: A {tuple(a.shape)}, W {tuple(w.shape)}, output {tuple(out.shape)}")
+    return library("fast").call_optional(
+        "bfi_gemm_tiles_bf16", _ptr(a), c_long(a.stride(0)), _ptr(w), c_long(w.stride(1)), c_long(w.stride(0)), c_int(groups), _ptr(tile_group),
+        _ptr(tiles_used), _ptr(out), c_int(dtype_code(out.dtype)), c_long(out.stride(0)), c_int(tiles), c_int(n), c_int(k), c_int(epilogue),
+        _ptr(tc_status(a.device)), _stream())
+
+
+def moe_combine(y: torch.Tensor, pair_row: torch.Tensor, weight, token_slot: torch.Tensor, out: torch.Tensor, shared=None, gate=None,
+                accumulate: bool = False) -> None:
+    """``out[t] (= | +=) sum_k weight[t, k] * y[pair_row[t, k]] + gate[t] * shared[t]``, all float32; ``weight`` and ``gate`` None are 1."""
+    _rows_2d(out, "feed-forward output")
+    n, width = out.shape
+    top = pair_row.shape[1]
+    if y.dtype != torch.float32 or not y.is_contiguous() or y.shape[1] != width or out.dtype != torch.float32 or pair_row.shape != (n, top) \
+            or pair_row.dtype != torch.int32 or not pair_row.is_contiguous():
+        raise KernelError("moe_combine: float32 rows of the output's width and int32 rows of pairs")
+    for t, least in ((weight, n * top), (gate, n)):
+        if t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or t.numel() < least):
+            raise KernelError("moe_combine: weights and gates are contiguous float32")
+    if shared is not None and (shared.dtype != torch.float32 or shared.shape != (n, width) or shared.stride(1) != 1):
+        raise KernelError("moe_combine: the shared output must be float32 [tokens, width]")
+    library("fast").call("bfi_moe_combine", _ptr(y), _ptr(pair_row), _ptr(weight), _ptr(shared), c_long(0 if shared is None else shared.stride(0)), _ptr(gate),
+                         _ptr(token_slot), c_int(n), c_int(top), c_int(width), _ptr(out), c_long(out.stride(0)), c_int(1 if accumulate else 0), _stream())

@@ -80,3 +80,22 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 
     elif a.dtype == w.dtype and a.shape[0] > SPLIT_MIN_ROWS and ops.gemm_split(a, w, out, epilogue):
         return
     ops.gemm_simt(a, w, out, epilogue)
+
+
+def linear_tiles(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, tiles_used: torch.Tensor, out: torch.Tensor,
+                 epilogue: int = EPI_STORE, gate=None, in_scale=None) -> bool:
+    """``linear`` for rows in tiles of 128 with a weight matrix each (``fast_ops.gemm_tiles``): ``w`` ``[groups, n, k]``, tile i takes
+    ``w[tile_group[i]]``.  ``gate`` as ``linear``'s; ``in_scale``: one float32 factor per row, with the gated epilogue."""
+    try:
+        if gate is not None:
+            _set_gate(True, *gate)
+        if in_scale is not None:
+            if epilogue != EPI_SWIGLU or in_scale.dtype != torch.float32 or in_scale.shape != (a.shape[0], 1) or not in_scale.is_contiguous():
+                raise ops.KernelError("linear_tiles: input factors are float32, one per row, for the gated epilogue")
+            _set_in_scale(True, in_scale, out.shape[1])
+        return _fast_ops().gemm_tiles(a, w, tile_group, tiles_used, out, epilogue)
+    finally:
+        if in_scale is not None:
+            _set_in_scale(True, None, 1)
+        if gate is not None:
+            _set_gate(True, 1.0, 0.0, 0.0)

@@ -1,0 +1,121 @@
+"""The routed feed-forward over rows sorted by expert: the sort, the products with a matrix per tile, and the whole part against a
+64-bit restatement, beside the dense way on the same step."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("n,top,E,skip", [(1, 1, 1, 0), (130, 4, 16, 3), (2048, 4, 16, 0), (700, 3, 300, 5), (5000, 2, 7, 1)])
+def test_sort_gives_every_pair_a_row_of_its_expert(n, top, E, skip):
+    from builderforce_inference_b200.kernels import fast_ops as f
+    g = torch.Generator(device=DEV).manual_seed(n)
+    idx = torch.rand(n, max(E, top), generator=g, device=DEV).argsort(1)[:, :top].int().contiguous()
+    if E > 2:
+        idx[idx == 2] = 0                                    # an expert nobody chose
+    slot = torch.zeros(n, dtype=torch.int32, device=DEV)
+    if skip:
+        slot[::skip + 1] = -1
+    tiles = f.moe_tiles(n * top, E)
+    pair_row, row_pair = torch.full((n, top), -7, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -7, dtype=torch.int32, device=DEV)
+    tile_expert, used = torch.full((tiles,), -7, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    f.moe_sort(idx, slot, E, pair_row, row_pair, tile_expert, used)
+    live = slot >= 0
+    counts = torch.bincount(idx[live].flatten().long(), minlength=E)
+    want = torch.repeat_interleave(torch.arange(E, device=DEV), (counts + 127) // 128)
+    assert int(used) == want.numel() <= tiles and torch.equal(tile_expert[:want.numel()].long(), want)
+    assert bool((pair_row[~live] == -1).all())
+    rows = pair_row[live].flatten().long()
+    assert rows.unique().numel() == rows.numel()
+    assert torch.equal(tile_expert[rows // 128], idx[live].flatten())
+    back = torch.arange(n * top, device=DEV).view(n, top)[live].flatten()
+    assert torch.equal(row_pair[rows].long(), back)
+    filler = torch.ones(int(used) * 128, dtype=torch.bool, device=DEV)
+    filler[rows] = False
+    assert bool((row_pair[:int(used) * 128][filler] == -1).all())
+
+
+@pytest.mark.parametrize("epilogue", [0, 2, 3])
+@pytest.mark.parametrize("E,N,K", [(3, 136, 72), (5, 512, 256), (2, 40, 8)])
+def test_tiles_with_a_matrix_each(epilogue, E, N, K):
+    from builderforce_inference_b200.kernels import fast_ops as f
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    group = torch.tensor([1, 0, E - 1, 0, 7], dtype=torch.int32, device=DEV)             # the last one is not used
+    a = torch.randn(5 * 128, K, generator=g, device=DEV).bfloat16()
+    wide = torch.randn(N, E * K + 8, generator=g, device=DEV).mul_(K ** -0.5).bfloat16()
+    w = wide.as_strided((E, N, K), (K, wide.stride(0), 1))                               # columns of a wider matrix, as the down matrices
+    cols = N // 2 if epilogue == 2 else N
+    out = torch.full((5 * 128, cols), 7.0, device=DEV)
+    assert f.gemm_tiles(a, w, group, torch.tensor([4], dtype=torch.int32, device=DEV), out, epilogue)
+    ref = torch.cat([a[i * 128:(i + 1) * 128].double() @ w[int(group[i])].double().T for i in range(4)])
+    if epilogue == 2:
+        ref = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
+    elif epilogue == 3:
+        ref = ref.clamp(min=0).square()
+    assert float((out[:512].double() - ref).norm() / ref.norm()) < 2e-6
+    assert bool((out[512:] == 7.0).all()) and int(f.tc_status(DEV)[0].item()) == 0
+
+
+def plain(kw, w, h, idx, wts, gate, padding):
+    f = lambda z: torch.nn.functional.silu(z)  # noqa: E731
+    limit = kw.get("limit")
+
+    def expert(p, x, scale=None):
+        u = x @ w[p + "up_proj"].T
+        if kw.get("expert") == "relu_squared":
+            return u.clamp(min=0).square() @ w[p + "down_proj"].T
+        g = x @ w[p + "gate_proj"].T
+        if scale is not None:
+            g, u = g * scale, u * scale
+        if limit:
+            g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+        return (f(g) * u) @ w[p + "down_proj"].T
+
+    y = torch.zeros_like(h)
+    for t in set(range(h.shape[0])) - {padding}:      # a padding row has no choices
+        for k in range(idx.shape[1]):
+            p = f"experts.{int(idx[t, k])}."
+            if kw.get("weight_on") == "input":
+                y[t] += expert(p, h[t:t + 1], wts[t, k])[0]
+            else:
+                y[t] += wts[t, k] * expert(p, h[t:t + 1])[0]
+    if kw.get("shared_inner"):
+        s = expert("shared.", h)
+        y += s * gate[:, None] if gate is not None else s
+    return y
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("kw", [dict(inner=40, shared_inner=56, n_groups=4, keep_groups=2),
+                                dict(inner=48, shared_inner=32, correction=False, score="sigmoid", expert="relu_squared", shared_gate=False),
+                                dict(inner=72, weight_on="input", limit=7.0, weight_scale=1.5), dict(inner=200)])
+def test_part_sorted_and_dense(kw, accumulate, monkeypatch):
+    from builderforce_inference_b200.engine.context import Workspace, build_context
+    from builderforce_inference_b200.engine.decoder import Runtime
+    from builderforce_inference_b200.parts import FEED_FORWARDS, PartSpec
+    from builderforce_inference_b200.parts import moe
+    n = 150
+    part = FEED_FORWARDS.build(PartSpec("mixture_of_experts", dict(width=72, n_experts=16, top=3, **kw)))
+    g = torch.Generator(device=DEV).manual_seed(3)
+    w = {k: (torch.randn(ps.shape, generator=g, device=DEV) * ps.shape[-1] ** -0.5).bfloat16() for k, ps in part.all_param_specs().items()}
+    part.load_all(w, Runtime(DEV, torch.bfloat16))
+    h = torch.randn(n, 72, generator=g, device=DEV).bfloat16()
+    ws = Workspace(DEV)
+    ctx = build_context([(0, 0, range(n))], torch.bfloat16, ws, DEV)
+    ctx.token_slot[5] = -1                                   # a padding row: left as it is
+    assert part._sorts(h, n)
+    old = torch.randn(n, 72, generator=g, device=DEV)
+    out = {}
+    for way in (True, False):
+        monkeypatch.setattr(moe, "SORTED_MIN_TOKENS", 1 if way else 1 << 30)
+        out[way] = old.clone()
+        (part.forward if accumulate else part.forward_store)(ctx, h, out[way])
+    idx, wts = ctx.rows("moe.idx", 3, torch.int32), ctx.rows("moe.weight", 3, torch.float32)
+    gate = ctx.rows("moe.gate", 1, torch.float32).view(-1).double() if part.shared_gate else None
+    ref = plain(dict(kw), {k: v.double() for k, v in w.items()}, h.double(), idx, wts.double(), gate, 5) + (old.double() if accumulate else 0.0)
+    keep = torch.ones(n, dtype=torch.bool, device=DEV)
+    keep[5] = False
+    assert torch.equal(out[True][5], old[5])
+    errs = {way: float((out[way][keep].double() - ref[keep]).norm() / ref[keep].norm()) for way in out}
+    assert errs[True] < 8e-3 and errs[True] <= errs[False] * 1.05
