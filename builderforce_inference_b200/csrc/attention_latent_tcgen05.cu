@@ -1,0 +1,429 @@
+// Latent attention over prompts (bfloat16) on the fifth-generation tensor cores: the function of attention_latent.cu for steps
+// with many query rows.  The cache holds one row of `d` = 128 NB + 64 values per token, whose first 128 NB are also its value;
+// the (token, head) pairs of a sequence are stacked, head fastest, into query rows, and 128 consecutive ones are a work item.
+//
+// The output of 128 rows x 512 values would fill the tensor memory of an SM by itself, and 128 query rows of 576 values most of its
+// shared memory.  So a cluster of two blocks shares an item and splits the VALUES of a row between them: block c has
+// columns [64 NB c, 64 NB (c + 1)) of the latent and half of the rotated part.  Its scores are then partial sums, which the two
+// exchange through each other's shared memory and add (the same two numbers, so both have the same scores, weights and
+// sums); its columns are exactly the values it needs for its half of the output.  Nothing is computed twice but the softmax.
+//   warps 0-3  softmax: a thread owns a row.  Partial scores of a tile of 64 keys out of tensor memory, to the other block
+//              (st.async, counted by the receiving warp's barrier) and from it; mask, running maximum (raised only when a
+//              score would exceed it by 2^8; the row of the output is then rescaled in tensor memory), exponentials; the weights
+//              go back over the scores as TWO bfloat16 terms, so that they stay float32 in effect.  At the end the row,
+//              divided by its sum and multiplied by the head's gate, out through shared memory as whole lines.
+//   warp 4     TMA: the item's query rows, then one page of keys at a time through a ring of three
+//   warp 5     one lane issues tcgen05.mma: the next tile's scores ahead of this tile's weighted values, so that the tensor
+//              cores work while the softmax does
+//
+// What bounds it: the tensor pipe, which takes 130 to 190 cycles an instruction here: 18 of 128 x 64 for a tile's scores and 8
+// of 128 x 256 for both terms of its weighted values, of each of the two blocks; the softmax with its exchange runs beside them.
+// 2,048 tokens, 16 heads of 576 values: @@.
+//
+// Every wait is bounded: one that runs out records BFI_STATUS_TIMEOUT, every role leaves its loop and the blocks return.
+#include "attention_tc.cuh"
+
+#define LT_ROWS 128
+#define LT_KEYS BFI_PAGE_TOKENS
+#define LT_STAGES 3
+#define LT_THREADS 192
+#define LT_RESCALE_ABOVE 8.0f
+#define LT_LOG2E 1.4426950408889634f
+#define LT_O_COL (2 * LT_KEYS)               // tensor memory: two score buffers, then the output
+#define LT_X_BYTES (32 * LT_KEYS * 4)        // a warp's partial scores
+
+template <int NB>
+struct LtConfig {
+    static constexpr int Q_BYTES = NB * LT_ROWS * 128 + LT_ROWS * 64;       // NB boxes of 64 values and one of 32
+    static constexpr int K_BYTES = NB * LT_KEYS * 128 + LT_KEYS * 64;
+    static constexpr int X_OFF = Q_BYTES + LT_STAGES * K_BYTES;
+    static constexpr int BAR_OFF = X_OFF + 4 * LT_X_BYTES;
+    static constexpr size_t SMEM = (size_t)BAR_OFF + 256 + 1024;
+    static_assert(4 * 32 * NB * 128 <= LT_STAGES * K_BYTES, "the output leaves through the ring");
+};
+
+__device__ __forceinline__ uint32_t lt_peer(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// 16 bytes into the other block's shared memory, counted by a barrier there.
+__device__ __forceinline__ void lt_send(uint32_t addr, const float* v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void lt_arrive_remote(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// A bounded wait that also acquires what the other block released.
+__device__ __forceinline__ bool lt_wait_cluster(uint64_t* bar, uint32_t parity, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void lt_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// grid (2 x tiles of 128 rows, sequences), clusters of two blocks along x
+template <int NB>
+__global__ void __launch_bounds__(LT_THREADS, 1)
+attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_rot,
+                           const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_k_rot, bf16* __restrict__ out,
+                           long out_stride, const int* __restrict__ block_table, int table_stride, const int* __restrict__ cu_seqlens,
+                           const int* __restrict__ seq_slot, const int* __restrict__ seq_start, int heads, float scale_log2,
+                           const float* __restrict__ sinks, const bf16* __restrict__ gate, long gate_stride, int* __restrict__ status) {
+    using Cfg = LtConfig<NB>;
+    const uint32_t spin_limit = TC_SPIN_LIMIT;
+    constexpr uint32_t FULL = 0xffffffffu;
+    pdl_trigger();
+    const int seq = blockIdx.y, slot = seq_slot[seq];
+    if (slot < 0) return;
+    const int t0 = cu_seqlens[seq], nt = cu_seqlens[seq + 1] - t0;
+    const long n_rows = (long)nt * heads;
+    const uint32_t rank = blockIdx.x & 1;
+    const long row0 = (long)((gridDim.x >> 1) - 1 - (blockIdx.x >> 1)) * LT_ROWS;      // the last rows walk the most keys: they start first
+    if (row0 >= n_rows) return;                                                        // the same for both blocks of the cluster
+    const int start = seq_start[seq], seq_hi = start + nt - 1;
+    const int hi_block = start + (int)((min(row0 + LT_ROWS, n_rows) - 1) / heads);
+    const int n_tiles = hi_block / LT_KEYS + 1;
+    const int* table = block_table + (size_t)slot * table_stride;
+
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char *q_smem = smem, *k_smem = smem + Cfg::Q_BYTES, *x_smem = smem + Cfg::X_OFF;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);
+    uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = k_full + LT_STAGES, *s_full = k_empty + LT_STAGES, *p_full = s_full + 2,
+             *o_tile = p_full + 2, *o_last = o_tile + 1, *x_full = o_last + 1, *x_empty = x_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_empty + 4);
+    volatile int* s_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        for (int s = 0; s < LT_STAGES; ++s) mbar_init(&k_full[s], 1), mbar_init(&k_empty[s], 1);
+        for (int s = 0; s < 2; ++s) mbar_init(&s_full[s], 1), mbar_init(&p_full[s], LT_ROWS);
+        mbar_init(o_tile, 1);                          // a phase per tile
+        mbar_init(o_last, 1);                          // the item's last one: nobody follows every phase of the other
+        for (int w = 0; w < 4; ++w) mbar_init(&x_full[w], 1), mbar_init(&x_empty[w], 1);
+        *s_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    lt_cluster_sync();                                 // both blocks' barriers exist
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+
+    if (warp == 4) {
+        // ---------------------------------------------------------------- TMA
+        if (lane == 0) {
+            const int col = (int)rank * NB * 64, col_rot = NB * 128 + (int)rank * 32;
+            const int q_row = (int)((long)t0 * heads + row0);
+            mbar_expect_tx(q_full, Cfg::Q_BYTES);
+            for (int b = 0; b < NB; ++b) tma_load_2d(q_smem + b * LT_ROWS * 128, &map_q, col + b * 64, q_row, q_full);
+            tma_load_2d(q_smem + NB * LT_ROWS * 128, &map_q_rot, col_rot, q_row, q_full);
+            for (int t = 0; t < n_tiles && !*s_flag; ++t) {
+                const int s = t % LT_STAGES;
+                const int page = max(table[t], 0);     // a page that does not exist: masked and cleared by the softmax warps
+                if (t >= LT_STAGES && !MBAR_WAIT(&k_empty[s], ((uint32_t)(t / LT_STAGES) & 1) ^ 1)) {
+                    atomicOr(status, BFI_STATUS_TIMEOUT);
+                    *s_flag = 1;
+                    break;
+                }
+                unsigned char* stage = k_smem + s * Cfg::K_BYTES;
+                mbar_expect_tx(&k_full[s], Cfg::K_BYTES);
+                for (int b = 0; b < NB; ++b) tma_load_2d(stage + b * LT_KEYS * 128, &map_k, col + b * 64, page * LT_KEYS, &k_full[s]);
+                tma_load_2d(stage + NB * LT_KEYS * 128, &map_k_rot, col_rot, page * LT_KEYS, &k_full[s]);
+            }
+        }
+    } else if (warp == 5) {
+        // ---------------------------------------------------------------- tensor-core issuer
+        if (lane == 0) {
+            constexpr uint32_t idesc_s = umma_idesc(LT_ROWS, LT_KEYS);
+            constexpr uint32_t idesc_o = umma_idesc_b_mn(LT_ROWS, NB * 64);
+            const uint32_t q_addr = smem_u32(q_smem), k_addr = smem_u32(k_smem);
+            bool ok = MBAR_WAIT(q_full, 0);
+            auto issue_s = [&](int t) {
+                const uint32_t k = k_addr + (t % LT_STAGES) * Cfg::K_BYTES, s_addr = tmem_base + (t & 1) * LT_KEYS;
+#pragma unroll
+                for (int kk = 0; kk < NB * 4; ++kk)
+                    umma_bf16(s_addr, umma_desc_sw128(q_addr + (kk >> 2) * LT_ROWS * 128 + (kk & 3) * 32),
+                              umma_desc_sw128(k + (kk >> 2) * LT_KEYS * 128 + (kk & 3) * 32), idesc_s, kk > 0);
+#pragma unroll
+                for (int kk = 0; kk < 2; ++kk)
+                    umma_bf16(s_addr, umma_desc_sw64(q_addr + NB * LT_ROWS * 128 + kk * 32), umma_desc_sw64(k + NB * LT_KEYS * 128 + kk * 32),
+                              idesc_s, 1u);
+                umma_commit(&s_full[t & 1]);
+            };
+            for (int t = 0; ok && t <= n_tiles && !*s_flag; ++t) {
+                if (t < n_tiles) {                     // the scores of tile t; P of tile t - 2, whose buffer this is, has been multiplied
+                    if (!MBAR_WAIT(&k_full[t % LT_STAGES], (uint32_t)(t / LT_STAGES) & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    issue_s(t);
+                }
+                if (t == 0) continue;
+                const int u = t - 1;                   // the weighted values of the tile before
+                if (!MBAR_WAIT(&p_full[u & 1], (uint32_t)(u >> 1) & 1)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t p_addr = tmem_base + (u & 1) * LT_KEYS;
+                const uint64_t v = umma_desc_mn_sw128(k_addr + (u % LT_STAGES) * Cfg::K_BYTES, LT_KEYS * 128, 1024);
+#pragma unroll
+                for (int term = 0; term < 2; ++term)
+#pragma unroll
+                    for (int kk = 0; kk < LT_KEYS / 16; ++kk)        // 16 keys: 8 columns of packed weights, 2048 bytes of a box
+                        umma_bf16_a_tmem(tmem_base + LT_O_COL, p_addr + term * (LT_KEYS / 2) + kk * 8, v + (uint64_t)(kk * 2048 >> 4), idesc_o,
+                                         (u > 0 || term > 0 || kk > 0));
+                umma_commit(&k_empty[u % LT_STAGES]);
+                umma_commit(o_tile);
+                if (t == n_tiles) umma_commit(o_last);
+            }
+            if (!ok) {
+                atomicOr(status, BFI_STATUS_TIMEOUT);
+                *s_flag = 1;
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- softmax and output
+        const long r = row0 + threadIdx.x;
+        const bool live = r < n_rows;
+        const int tok = live ? (int)(r / heads) : 0, h = live ? (int)(r - (long)tok * heads) : 0;
+        const int pos = live ? start + tok : -1;
+        const int pos_first = start + (int)(row0 / heads);         // no row of the item sees less
+        const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const uint32_t o_addr = lane_base + LT_O_COL;
+        const uint32_t x_own = smem_u32(x_smem) + warp * LT_X_BYTES + lane * 16;         // [16 groups of 4 keys][32 rows][4]
+        const uint32_t x_peer = lt_peer(x_own, rank ^ 1), full_peer = lt_peer(smem_u32(&x_full[warp]), rank ^ 1),
+                       empty_peer = lt_peer(smem_u32(&x_empty[warp]), rank ^ 1);
+        float m_used = -INFINITY, l_run = 0.0f;
+        bool ok = true;
+        int page = table[0];
+        for (int t = 0; t < n_tiles; ++t) {
+            const uint32_t b = t & 1;
+            const bool have = page >= 0;
+            if (t + 1 < n_tiles) page = table[t + 1];
+            if (__any_sync(FULL, *s_flag != 0)) { ok = false; break; }
+            if (!__all_sync(FULL, MBAR_WAIT(&s_full[b], (uint32_t)(t >> 1) & 1))) { ok = false; break; }
+            tc_fence_after();
+            float s[LT_KEYS];
+            const uint32_t s_addr = lane_base + b * LT_KEYS;
+            tmem_ld32(s_addr, s);
+            tmem_ld32(s_addr + 32, s + 32);
+            tmem_wait_ld();
+            // the other half of the sums: ours to the other block, which has read those of the tile before; its to us
+            if (lane == 0) mbar_expect_tx(&x_full[warp], LT_X_BYTES);
+            if (t > 0 && !__all_sync(FULL, lt_wait_cluster(&x_empty[warp], (uint32_t)(t - 1) & 1, spin_limit))) { ok = false; break; }
+#pragma unroll
+            for (int e = 0; e < LT_KEYS; e += 4) lt_send(x_peer + e * 128, s + e, full_peer);
+            if (!__all_sync(FULL, lt_wait_cluster(&x_full[warp], (uint32_t)t & 1, spin_limit))) { ok = false; break; }
+#pragma unroll
+            for (int e = 0; e < LT_KEYS; e += 4) {
+                const uint4 x = lds128(x_own + e * 128);
+                s[e] += __uint_as_float(x.x), s[e + 1] += __uint_as_float(x.y), s[e + 2] += __uint_as_float(x.z), s[e + 3] += __uint_as_float(x.w);
+            }
+            __syncwarp();
+            if (lane == 0) lt_arrive_remote(empty_peer);
+
+            const int key0 = t * LT_KEYS;
+            if (!have || key0 + LT_KEYS - 1 > pos_first) {
+                const int hi = have ? pos - key0 : -1;
+#pragma unroll
+                for (int e = 0; e < LT_KEYS; ++e) s[e] = e > hi ? -INFINITY : s[e];
+            }
+            float mx = s[0];
+#pragma unroll
+            for (int e = 1; e < LT_KEYS; ++e) mx = fmaxf(mx, s[e]);
+            // raise the running maximum only when a weight would otherwise exceed 2^8
+            const bool raise = mx > -INFINITY && (m_used == -INFINITY || (mx - m_used) * scale_log2 > LT_RESCALE_ABOVE);
+            if (__any_sync(FULL, raise && t > 0)) {
+                const float m_new = raise ? mx : m_used;
+                const float f = (raise && m_used > -INFINITY) ? ft_exp2((m_used - m_new) * scale_log2) : 1.0f;
+                // (the scores of tile t came behind the products of tile t - 2, so this is the phase of t - 1 and no other)
+                if (!__all_sync(FULL, MBAR_WAIT(o_tile, (uint32_t)(t - 1) & 1))) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < NB * 2; ++c) {
+                    float o[32];
+                    uint32_t ou[32];
+                    tmem_ld32(o_addr + c * 32, o);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) ou[e] = __float_as_uint(o[e] * f);
+                    tmem_st32(o_addr + c * 32, ou);
+                }
+                l_run *= f;
+                m_used = m_new;
+            } else if (raise) {
+                m_used = mx;                           // the first tile: nothing accumulated yet
+            }
+            const float mc = m_used == -INFINITY ? 0.0f : m_used * scale_log2;
+            float sum = 0.0f;
+            uint32_t ph[32], pl[32];
+#pragma unroll
+            for (int e = 0; e < LT_KEYS; e += 2) {
+                const float a = ft_exp2(fmaf(s[e], scale_log2, -mc)), c = ft_exp2(fmaf(s[e + 1], scale_log2, -mc));
+                sum += a + c;
+                const uint32_t p2 = ft_pack(a, c);
+                ph[e >> 1] = p2;
+                pl[e >> 1] = ft_pack(a - __uint_as_float(p2 << 16), c - __uint_as_float(p2 & 0xffff0000u));
+            }
+            tmem_st32(s_addr, ph);
+            tmem_st32(s_addr + 32, pl);
+            l_run += sum;
+            // rows that the cache never wrote: zeros, so that a weight of zero cannot meet a stray NaN
+            const int first_bad = have ? seq_hi + 1 - key0 : 0;
+            if (first_bad < LT_KEYS) {
+                unsigned char* stage = k_smem + (t % LT_STAGES) * Cfg::K_BYTES;
+                const int bytes = (LT_KEYS - first_bad) * 128;
+                for (int x = threadIdx.x * 16; x < NB * bytes; x += LT_ROWS * 16) {
+                    const int box = x / bytes, off = x - box * bytes;
+                    *reinterpret_cast<uint4*>(stage + box * LT_KEYS * 128 + first_bad * 128 + off) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                fence_proxy_async_smem();
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(&p_full[b]);
+        }
+        ok = ok && __all_sync(FULL, MBAR_WAIT(o_last, 0));
+        if (ok) {
+            tc_fence_after();
+            float l = l_run;
+            if (sinks != nullptr && m_used > -INFINITY) l += ft_exp2(sinks[h] * LT_LOG2E - m_used * scale_log2);
+            float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            if (gate != nullptr && live) inv *= 1.0f / (1.0f + expf(-__bfloat162float(gate[(size_t)(t0 + tok) * gate_stride + h])));
+            const uint32_t stage = smem_u32(k_smem) + warp * 32 * NB * 128;               // [32 rows][NB x 128 bytes]
+#pragma unroll
+            for (int c = 0; c < NB * 2; ++c) {
+                float o[32];
+                tmem_ld32(o_addr + c * 32, o);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 32; e += 8) {
+                    const uint4 w = make_uint4(ft_pack(o[e] * inv, o[e + 1] * inv), ft_pack(o[e + 2] * inv, o[e + 3] * inv),
+                                               ft_pack(o[e + 4] * inv, o[e + 5] * inv), ft_pack(o[e + 6] * inv, o[e + 7] * inv));
+                    sts128(stage + lane * NB * 128 + (((c * 4 + (e >> 3)) ^ (lane & 7)) << 4), w);
+                }
+            }
+            __syncwarp();
+            const long my_off = (long)(t0 + tok) * out_stride + (long)h * (NB * 128) + (long)rank * (NB * 64);
+#pragma unroll 4
+            for (int i = 0; i < NB * 8; ++i) {
+                const int piece = i * 32 + lane, row = piece / (NB * 8), p = piece - row * (NB * 8);
+                const long off = __shfl_sync(FULL, my_off, row);
+                const bool on = __shfl_sync(FULL, live, row);
+                const uint4 w = lds128(stage + row * NB * 128 + ((p ^ (row & 7)) << 4));
+                if (on) *reinterpret_cast<uint4*>(out + off + p * 8) = w;
+            }
+        } else {
+            if (lane == 0) {
+                atomicOr(status, BFI_STATUS_TIMEOUT);
+                *s_flag = 1;
+            }
+            // give what the other block may still be sending a bounded time to land
+            lt_wait_cluster(&x_full[warp], 0, spin_limit >> 4), lt_wait_cluster(&x_full[warp], 1, spin_limit >> 4);
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (*s_flag && warp == 4 && lane == 0) {
+        // a wait ran out: give outstanding TMA writes a bounded time to land
+        MBAR_WAIT(q_full, 0);
+        for (int s = 0; s < LT_STAGES; ++s) MBAR_WAIT(&k_full[s], 0), MBAR_WAIT(&k_full[s], 1);
+    }
+    __syncthreads();
+    if (warp == 5) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+    __syncwarp();
+    lt_cluster_sync();                                 // no block may leave while the other still writes to it
+    BFI_TRACE_END();
+}
+
+template <int NB>
+static int launch_latent_tc(const void* q, long q_rows, void* out, long out_stride, const void* pages, long n_pages, const int* block_table,
+                            int table_stride, const int* cu_seqlens, const int* seq_slot, const int* seq_start, int n_seqs, int max_tokens,
+                            int heads, float scale, const float* sinks, const bf16* gate, long gate_stride, int* status, cudaStream_t stream) {
+    constexpr int d = NB * 128 + 64;
+    using Cfg = LtConfig<NB>;
+    auto kernel = attention_latent_tc_kernel<NB>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+        if (e != cudaSuccess) return bfi_fail("attention_latent_tcgen05: cannot reserve %zu bytes of shared memory: %s", Cfg::SMEM, cudaGetErrorString(e));
+        configured = true;
+    }
+    CUtensorMap mq, mqr, mk, mkr;
+    int rc = bfi_tensor_map_groups_bf16(q, q_rows, d, d, 0, 0, LT_ROWS, &mq);
+    if (!rc) rc = bfi_tensor_map_groups_bf16(q, q_rows, d, d, 0, 0, LT_ROWS, &mqr, 32);
+    if (!rc) rc = bfi_tensor_map_groups_bf16(pages, n_pages * LT_KEYS, d, d, 0, 0, LT_KEYS, &mk);
+    if (!rc) rc = bfi_tensor_map_groups_bf16(pages, n_pages * LT_KEYS, d, d, 0, 0, LT_KEYS, &mkr, 32);
+    if (rc) return rc;
+    const long tiles = ((long)max_tokens * heads + LT_ROWS - 1) / LT_ROWS;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * tiles), n_seqs);
+    cfg.blockDim = dim3(LT_THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_bfi_pdl ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mq, mqr, mk, mkr, (bf16*)out, out_stride, block_table, table_stride, cu_seqlens, seq_slot, seq_start,
+                                       heads, scale * LT_LOG2E, sinks, gate, gate_stride, status);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return bfi_fail("attention_latent_tcgen05: launch failed: %s", cudaGetErrorString(e));
+    }
+    return bfi_check_launch("attention_latent_tcgen05");
+}
+
+// The arguments of bfi_attention_latent_bf16 without key ranges, and the cache's number of pages (`n_tokens`: of the whole step).
+// Returns 2 when the shape is not taken (nothing launched): rows of 128, 256, 384 or 512 values and a rotated part of 64, stacked
+// without gaps.
+extern "C" int bfi_attention_latent_tcgen05_bf16(const void* q, long q_stride, void* out, long out_stride, const void* pages, long n_pages,
+                                                 const int* block_table, int table_stride, const int* cu_seqlens, const int* seq_slot,
+                                                 const int* seq_start, int n_seqs, int n_tokens, int max_tokens, int heads, int d, int dv,
+                                                 float scale, const float* sinks, const void* gate, long gate_stride, int* status,
+                                                 cudaStream_t stream) {
+    BFI_REQUIRE(heads > 0 && d > 0 && dv > 0 && dv <= d, "attention_latent_tcgen05: bad sizes heads=%d d=%d dv=%d", heads, d, dv);
+    BFI_REQUIRE(status != nullptr, "attention_latent_tcgen05: a status word is required");
+    if (n_seqs <= 0 || max_tokens <= 0) return 0;
+    if (d != dv + 64 || dv % 128 != 0 || dv > 512 || !(scale > 0.0f)) return 2;
+    if (q_stride != (long)heads * d || out_stride % 8 != 0 || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)pages & 15)) return 2;
+    if (n_seqs > 65535 || (long)n_tokens * heads > 0x7fffffffL || n_pages * LT_KEYS > 0x7fffffffL || (long)max_tokens * heads > (1L << 36)) return 2;
+#define BFI_LT(NB)                                                                                                                            \
+    return launch_latent_tc<NB>(q, (long)n_tokens * heads, out, out_stride, pages, n_pages, block_table, table_stride, cu_seqlens, seq_slot, seq_start, \
+                                n_seqs, max_tokens, heads, scale, sinks, (const bf16*)gate, gate_stride, status, stream)
+    switch (dv / 128) {
+        case 1: BFI_LT(1);
+        case 2: BFI_LT(2);
+        case 3: BFI_LT(3);
+        default: BFI_LT(4);
+    }
+#undef BFI_LT
+}
+
+BFI_TRACE_EXPORT(attention_latent_tcgen05)

@@ -29,7 +29,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "fast": ["errors.cu", "skinny_gemm.cu", "attention_decode.cu", "attention_prefill.cu", "gemm_tcgen05.cu",
              "attention_prefill_tcgen05.cu", "attention_latent.cu", "weight_stream.cu", "lightning_chunked.cu",
              "mlstm_chunked.cu", "decay_chunked.cu",
-             "moe_sorted.cu"],
+             "moe_sorted.cu", "attention_latent_tcgen05.cu"],
 }
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -55,17 +55,6 @@
 #define GS_SMEM ((size_t)GS_STAGES * GS_STAGE_BYTES + 1024 + 128)
 static_assert(GS_TOKENS * GS_OUT_LD * 4 <= GS_STAGES * GS_STAGE_BYTES, "the tile leaves through the ring");
 
-// K-major tile with 64-byte rows and the 64-byte swizzle: groups of 8 rows 512 bytes apart, layout type 4.
-__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(512 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)4 << 61;
-    return d;
-}
-
 // One output by float32 multiply-adds, k rising: for results that are not finite.
 __device__ __noinline__ float dot_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
     float s = 0.0f;

@@ -829,8 +829,10 @@ struct MapKey {
     long rows, cols, ld;
     int box_rows;
     long groups, step;
+    int box_cols;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && groups == o.groups && step == o.step;
+        return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && groups == o.groups && step == o.step &&
+               box_cols == o.box_cols;
     }
 };
 struct MapKeyHash {
@@ -841,6 +843,7 @@ struct MapKeyHash {
         h = h * 1000003u ^ std::hash<long>()(k.ld);
         h = h * 1000003u ^ std::hash<long>()(k.groups);
         h = h * 1000003u ^ std::hash<long>()(k.step);
+        h = h * 1000003u ^ std::hash<int>()(k.box_cols);
         return h * 1000003u ^ std::hash<int>()(k.box_rows);
     }
 };
@@ -852,8 +855,9 @@ int bfi_tensor_map_bf16(const void* ptr, long rows, long cols, long ld, int box_
 }
 
 // `groups` 0: a plain matrix (two coordinates).
-int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out) {
-    MapKey key{ptr, rows, cols, ld, box_rows, groups, step};
+int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out,
+                               int box_cols) {
+    MapKey key{ptr, rows, cols, ld, box_rows, groups, step, box_cols};
     std::lock_guard<std::mutex> lock(g_maps_mutex);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) {
@@ -864,11 +868,11 @@ int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, l
     if (!fn) return bfi_fail("gemm_tcgen05: the driver does not export cuTensorMapEncodeTiled");
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)groups};
     cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)step * 2};
-    cuuint32_t box[3] = {TC_BK, (cuuint32_t)box_rows, 1};
+    cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMap m;
     CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups > 0 ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return bfi_fail("gemm_tcgen05: cuTensorMapEncodeTiled failed with code %d", (int)r);
     if (g_maps.size() > 4096) g_maps.clear();

@@ -131,6 +131,17 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
     d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
     return d;
 }
+// K-major tile with 64-byte rows and the 64-byte swizzle: groups of 8 rows 512 bytes apart, layout type 4.
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
 // Instruction descriptor, kind::f16: D float32, A and B bfloat16, both K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -142,4 +153,6 @@ __host__ __device__ constexpr uint32_t umma_idesc(int m, int n) {
 int bfi_tensor_map_bf16(const void* ptr, long rows, long cols, long ld, int box_rows, CUtensorMap* out);
 // The same for `groups` such matrices, each `step` elements behind the one before: x, row, group.  What lies past a
 // group's columns or rows reads as zero, whatever the memory there holds.
-int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out);
+// `box_cols`: 64 with the 128-byte swizzle, or 32 with the 64-byte one.
+int bfi_tensor_map_groups_bf16(const void* ptr, long rows, long cols, long ld, long groups, long step, int box_rows, CUtensorMap* out,
+                               int box_cols = 64);

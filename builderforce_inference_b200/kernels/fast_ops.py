@@ -252,6 +252,7 @@ def attention_prefill_bf16(ctx, qkv: torch.Tensor, out: torch.Tensor, kv, n_head
         _ptr(sinks), c_int(1 if exact_weights else 0), c_float(softcap or 0.0), _stream())
 
 
+LATENT_TCGEN05_MIN_ROWS = 256   # query rows (tokens x heads) of a sequence from which the tcgen05 kernel takes a step
 LATENT_TILES_PER_RANGE = 4      # a key range of the latent attention is at least this many tiles of 32 keys
 
 
@@ -290,6 +291,12 @@ def attention_latent_bf16(ctx, q: torch.Tensor, out: torch.Tensor, kv, n_heads: 
         return False
     if gate is not None and (gate.dtype != torch.bfloat16 or gate.stride(1) != 1 or gate.shape[1] != n_heads):
         return False
+    if splits is None and ctx.max_seq_tokens * n_heads >= LATENT_TCGEN05_MIN_ROWS and out.stride(1) == 1 and library("fast").call_optional(
+            "bfi_attention_latent_tcgen05_bf16", _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(kv.k),
+            c_long(kv.k.shape[0]), _ptr(kv.block_table), c_int(kv.block_table.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.seq_slot),
+            _ptr(ctx.seq_start), c_int(ctx.n_seqs), c_int(q.shape[0]), c_int(ctx.max_seq_tokens), c_int(n_heads), c_int(d), c_int(dv),
+            c_float(scale), _ptr(sinks), _ptr(gate), c_long(gate.stride(0) if gate is not None else 0), _ptr(tc_status(q.device)), _stream()):
+        return True
     max_pages = kv.block_table.shape[1]
     bucket = getattr(ctx, "pages_bucket", 0)
     if bucket:
