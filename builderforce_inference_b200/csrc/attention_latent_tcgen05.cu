@@ -16,9 +16,12 @@
 //   warp 5     one lane issues tcgen05.mma: the next tile's scores ahead of this tile's weighted values, so that the tensor
 //              cores work while the softmax does
 //
-// What bounds it: the tensor pipe, which takes 130 to 190 cycles an instruction here: 18 of 128 x 64 for a tile's scores and 8
-// of 128 x 256 for both terms of its weighted values, of each of the two blocks; the softmax with its exchange runs beside them.
-// 2,048 tokens, 16 heads of 576 values: @@.
+// What bounds it: a tile takes 5,200 cycles (2.9 us), the chain of one softmax warp per scheduler: scores out of tensor memory,
+// the exchange's trip there and back, 64 exponentials, two terms back.  The tensor pipe beside it takes about 3,900 (18
+// instructions of 128 x 64 for the scores, 8 of 128 x 256 for the weighted values, 130 to 190 cycles each).
+// attention_latent.cu -> this kernel (values of 512 and 64 rotated, 16 heads):
+//     one prompt of 2,048 tokens: 560 -> 166 us     8,192 tokens: 8,024 -> 2,117 us     512 tokens: 83 -> 28 us
+//     16 pieces of 16 tokens behind 4,000 cached: 307 -> 169 us     one piece of 16 tokens: 16 -> 14 us
 //
 // Every wait is bounded: one that runs out records BFI_STATUS_TIMEOUT, every role leaves its loop and the blocks return.
 #include "attention_tc.cuh"

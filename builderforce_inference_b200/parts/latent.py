@@ -20,7 +20,7 @@ rows another layer's run has written, with its own ``W_uk`` and ``W_uv``.
 
 Launches: one product for queries, gate logits and down projection together; ``latent_prepare``
 (rotations, the latent's norm, the cache write); ``latent_absorb``; the attention (in bfloat16 the
-tensor-core kernel over stacked (token, head) rows, cut into key ranges when a step has few rows;
+tensor-core kernels over stacked (token, head) rows, tcgen05 for prompts, cut into key ranges when a step has few rows;
 otherwise the general paged kernel, and the gate then waits for ``latent_expand``);
 ``latent_expand`` (``W_uv`` and the gate); the output product, which adds into the residual stream.
 In bfloat16 (when every slice starts on 16 bytes) ``latent_absorb`` and ``latent_expand`` are tensor-core
