@@ -11,7 +11,7 @@ one head's rows of a page are contiguous.
 Storage of a key/value group: ``[runs, 2, pages, kv_heads, PAGE_TOKENS, head_dim]`` in the run
 dtype.  The page table ``[slots, blocks]`` (int32, -1 where no page is held) is mirrored on the
 device; kernels find position ``p`` of slot ``s`` at page ``table[s, p // PAGE_TOKENS]``, row
-``p % PAGE_TOKENS``.
+``p % PAGE_TOKENS``.  Rows that change (pages taken, given back) reach the device with the next step.
 
 Sizing follows the reference's arithmetic (crates/bfi-models/src/kv_plan.rs:49-51): bytes per
 token = runs * 2 * kv_heads * head_dim * element size.
@@ -25,6 +25,7 @@ import torch
 
 from ..parts.base import KVNeed, StateNeed
 from .pages import PAGE_TOKENS, CacheError, FreeList, PageTable
+from .staging import PinnedRings
 
 _TORCH_DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
 
@@ -97,6 +98,7 @@ class _KVGroup:
         self.table = PageTable(n_pages, need.window, need.chunk, need.keep_first)
         self.n_blocks = n_blocks
         self.device = device
+        self._staging = PinnedRings()
         self.storage = self.v_storage = None
         if need.values_in_keys:     # keys only: the values are read out of them
             self.storage = torch.empty((len(keys), 1, n_pages, need.n_kv_heads, PAGE_TOKENS, need.head_dim),
@@ -113,10 +115,9 @@ class _KVGroup:
         self._alloc_tables(n_slots)
 
     def _alloc_tables(self, n_slots: int) -> None:
-        # The host mirror is pageable on purpose: a copy from pageable memory is staged before
-        # the call returns, so a row may be edited again while earlier work is still queued.
         self.block_host = torch.full((n_slots, self.n_blocks), -1, dtype=torch.int32)
         self.block_dev = torch.full((n_slots, self.n_blocks), -1, dtype=torch.int32, device=self.device)
+        self.stale = set()                     # slots whose row on the device is not the host's
 
     def grow_slots(self, n_slots: int) -> None:
         old_host = self.block_host
@@ -125,14 +126,38 @@ class _KVGroup:
         self.block_dev.copy_(self.block_host)
 
     def sync_row(self, slot: int) -> None:
+        """The slot's row of the host's table, from its pages; the device's follows with the next step (``send_rows``)."""
         row = self.table.rows.get(slot, [])
-        host = self.block_host[slot]
-        host.fill_(-1)
+        host = self.block_host.numpy()[slot]
+        host.fill(-1)
         if row:
             if len(row) > self.n_blocks:
                 raise CacheError(f"slot {slot} needs {len(row)} page blocks, table has {self.n_blocks}")
-            host[:len(row)] = torch.tensor(row, dtype=torch.int32)
-        self.block_dev[slot].copy_(host)
+            host[:len(row)] = row
+        self.stale.add(slot)
+
+    def send_rows(self) -> None:
+        """The rows that have changed since the last step, to the device: one copy where they lie close together.  They go
+        through page-locked buffers, which the host does not wait for (a copy out of pageable memory first waits for
+        everything queued before it, once for every row)."""
+        if not self.stale:
+            return
+        slots = sorted(self.stale)
+        self.stale.clear()
+        first, last = slots[0], slots[-1]
+        spans = [(first, last + 1)] if last + 1 - first <= 4 * len(slots) + 16 else [(s, s + 1) for s in slots]
+        for lo, hi in spans:
+            rows = self.block_host[lo:hi]
+            if self.device.type != "cuda":
+                self.block_dev[lo:hi].copy_(rows)
+                continue
+            entry = self._staging.take(rows.numel())
+            pinned = entry[0][:rows.numel()].view(rows.shape)
+            pinned.copy_(rows)
+            self.block_dev[lo:hi].copy_(pinned, non_blocking=True)
+            if entry[1] is None:
+                entry[1] = torch.cuda.Event()
+            entry[1].record(torch.cuda.current_stream(self.device))
 
     def view(self, key, mask: Optional[KVNeed] = None) -> KVView:
         """``mask``: the need whose window, kept first positions and chunk the reader goes by (default:
@@ -336,6 +361,7 @@ class SequenceCache:
             for s, c in zip(slots, counts):
                 if g.table.ensure(s, self.lengths[s], self.lengths[s] + c):
                     g.sync_row(s)
+            g.send_rows()
 
     def end_step(self, slots: Sequence[int], counts: Sequence[int]) -> None:
         """The step ran: lengths advance, and windowed groups let go of pages behind the window."""

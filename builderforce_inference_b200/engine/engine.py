@@ -25,6 +25,7 @@ import torch
 from ..cache.cache import SequenceCache
 from ..cache.pages import PAGE_TOKENS, CacheError
 from ..cache.plan import plan_cache
+from ..cache.staging import PINNED_RING, PinnedRings  # noqa: F401  (part of this module's names)
 from ..config.base import read_json, stop_ids_of_folder
 from ..kernels import ops
 from ..kernels.library import total_calls
@@ -34,8 +35,6 @@ from ..weights.loader import load_folder
 from ..weights.random_init import random_tensors
 from .context import StepContext, Workspace
 from .decoder import Decoder, Runtime, expected_tensors
-
-PINNED_RING = 4          # pinned staging buffers per size of a step's index arrays
 
 
 def pack_meta(dst: np.ndarray, tok, pos, slot_of, cu, n_tok: int, n_seq: int, seq_slots, seq_starts, pages: int,
@@ -69,41 +68,6 @@ def pack_meta(dst: np.ndarray, tok, pos, slot_of, cu, n_tok: int, n_seq: int, se
     dst[o:o + len(want_rows)] = want_rows
     return o + len(want_rows)
 
-
-
-class PinnedRings:
-    """Page-locked staging buffers for the steps' index arrays: ``PINNED_RING`` buffers in rotation
-    per capacity, capacities being powers of two (at least ``MIN_CAPACITY`` values).  However many
-    distinct lengths are asked for, at most ``PINNED_RING * log2(largest / MIN_CAPACITY)`` buffers
-    ever exist.  An entry is ``[buffer, event]``; ``take`` waits for the event of the entry it hands
-    out, so a buffer is never rewritten while a copy still reads it."""
-
-    MIN_CAPACITY = 64
-
-    def __init__(self, make=None):
-        self._rings: Dict[int, dict] = {}
-        self._make = make or (lambda cap: torch.empty(cap, dtype=torch.int32, pin_memory=True))
-
-    @classmethod
-    def capacity_for(cls, n: int) -> int:
-        cap = cls.MIN_CAPACITY
-        while cap < n:
-            cap *= 2
-        return cap
-
-    def take(self, n: int) -> list:
-        ring = self._rings.setdefault(self.capacity_for(n), {"next": 0, "slots": []})
-        if len(ring["slots"]) < PINNED_RING:
-            ring["slots"].append([self._make(self.capacity_for(n)), None])
-            return ring["slots"][-1]
-        entry = ring["slots"][ring["next"]]
-        ring["next"] = (ring["next"] + 1) % PINNED_RING
-        if entry[1] is not None:
-            entry[1].synchronize()
-        return entry
-
-    def n_buffers(self) -> int:
-        return sum(len(r["slots"]) for r in self._rings.values())
 
 
 DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32, "fp32": torch.float32}
