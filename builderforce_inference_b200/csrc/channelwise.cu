@@ -22,12 +22,6 @@
 #define SCAN_CAND_POSITIVE 1
 #define SCAN_MAX_WARPS 32
 
-__device__ __forceinline__ float cw_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
-
 struct ScanArgs {
     long p_stride, y_stride;
     int z_off, u_off, g_off;        // g_off < 0: no output gate
@@ -39,7 +33,7 @@ struct ScanArgs {
 // float32 arithmetic in both; with bfloat16 projections the exponential and the division are the hardware's
 // approximations (a few units in the last place of a float32, far below what the projections' rounding left)
 template <typename T>
-__device__ __forceinline__ float scan_sigmoid(float x) { return cw_sigmoid(x); }
+__device__ __forceinline__ float scan_sigmoid(float x) { return sigmoid_f32(x); }
 template <>
 __device__ __forceinline__ float scan_sigmoid<bf16>(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 
@@ -272,7 +266,7 @@ __global__ void sigmoid_gate_kernel(T* __restrict__ x, long x_stride, const T* _
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cols) return;
     T* p = x + (size_t)t * x_stride + j;
-    *p = from_f32<T>(to_f32(*p) * cw_sigmoid(to_f32(g[(size_t)t * g_stride + j / group])));
+    *p = from_f32<T>(to_f32(*p) * sigmoid_f32(to_f32(g[(size_t)t * g_stride + j / group])));
 }
 
 // bfloat16 rows in whole groups of 8 values that share a gate or have one each

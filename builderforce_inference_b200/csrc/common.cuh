@@ -222,17 +222,17 @@ __device__ __forceinline__ float relu_squared(float v) {
     return v * v;
 }
 
+// sigmoid(x) = 1 / (1 + e^-x) = e^x / (1 + e^x), whichever has the exponential that cannot overflow: one exponential of -|x|
+// and one division, without a branch that a warp's values would take both ways.
+__device__ __forceinline__ float sigmoid_f32(float x) {
+    const float e = expf(-fabsf(x));
+    return (x >= 0.0f ? 1.0f : e) / (1.0f + e);
+}
+
 // 0.5 g (1 + tanh(y)) = g * sigmoid(2 y): one exponential, no cancellation for large |y|
 __device__ __forceinline__ float gelu_tanh_exact(float g) {
     const float y = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    float s;
-    if (y >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-2.0f * y));
-    } else {
-        const float e = expf(2.0f * y);
-        s = e / (1.0f + e);
-    }
-    return g * s;
+    return g * sigmoid_f32(2.0f * y);
 }
 
 __device__ __forceinline__ float gate_mul_exact(float g, float u, const GateAct a) {
@@ -241,15 +241,7 @@ __device__ __forceinline__ float gate_mul_exact(float g, float u, const GateAct 
         g = fminf(g, a.limit);
         u = fminf(fmaxf(u, -a.limit), a.limit);
     }
-    const float z = a.alpha * g;
-    float s;                       // overflow-safe two-branch sigmoid
-    if (z >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-z));
-    } else {
-        const float e = expf(z);
-        s = e / (1.0f + e);
-    }
-    return g * s * (u + a.shift);
+    return g * sigmoid_f32(a.alpha * g) * (u + a.shift);
 }
 __device__ __forceinline__ float gate_mul_fast(float g, float u, const GateAct a) {
     if (a.kind == BFI_GATE_GELU_TANH) {

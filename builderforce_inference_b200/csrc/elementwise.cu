@@ -178,17 +178,7 @@ extern "C" int bfi_rmsnorm(const void* x, int x_dtype, long x_stride, const int*
 // SiLU(gate) * up.  `interleaved` != 0: the input row holds gate_j, up_j at columns 2j, 2j+1;
 // otherwise gate fills the first half of the row and up the second.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ float silu_f32(float g) {
-    // overflow-safe two-branch sigmoid, as the reference evaluates it
-    float s;
-    if (g >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-g));
-    } else {
-        const float z = expf(g);
-        s = z / (1.0f + z);
-    }
-    return g * s;
-}
+__device__ __forceinline__ float silu_f32(float g) { return g * sigmoid_f32(g); }
 
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, long in_stride, T* __restrict__ out, long out_stride,
@@ -214,15 +204,7 @@ __device__ __forceinline__ float gate_mul_f32(float g, float u, float alpha, flo
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit);
     }
-    const float z = alpha * g;
-    float s;
-    if (z >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-z));
-    } else {
-        const float e = expf(z);
-        s = e / (1.0f + e);
-    }
-    return g * s * (u + shift);
+    return g * sigmoid_f32(alpha * g) * (u + shift);
 }
 
 template <typename T>

@@ -17,17 +17,6 @@
 #define EPI_ACCUMULATE 1
 #define EPI_SWIGLU 2
 
-__device__ __forceinline__ float silu_mul_f32(float g, float u) {
-    float s;
-    if (g >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-g));
-    } else {
-        const float z = expf(g);
-        s = z / (1.0f + z);
-    }
-    return g * s * u;
-}
-
 // ------------------------------------------------------------------------------------------
 // Tiled kernel: 64x64 output tile, K step 16, 256 threads, 4x4 outputs per thread.
 // ------------------------------------------------------------------------------------------

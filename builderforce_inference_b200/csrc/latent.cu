@@ -194,11 +194,6 @@ extern "C" int bfi_latent_absorb(const void* proj, int dtype, long proj_stride, 
 // its head as float32; a warp owns ONE output row i of the head and walks W_uv's row once for all
 // staged tokens.  Few tokens still make heads * dv / 8 blocks.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ float lat_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
 
 template <typename T, typename TW>
 __global__ void __launch_bounds__(LAT_THREADS)
@@ -220,7 +215,7 @@ latent_expand_kernel(const T* __restrict__ lat, long lat_stride, const TW* __res
         const int t = t0 + threadIdx.x;
         float g = 1.0f;
         if (gate != nullptr && !gate_values && t < n_tokens && token_slot[t] >= 0)
-            g = lat_sigmoid(to_f32(gate[(size_t)t * gate_stride + h]));
+            g = sigmoid_f32(to_f32(gate[(size_t)t * gate_stride + h]));
         gs[threadIdx.x] = g;
     }
     __syncthreads();
@@ -245,7 +240,7 @@ latent_expand_kernel(const T* __restrict__ lat, long lat_stride, const TW* __res
                 if (t < n_tokens && token_slot[t] >= 0) {
                     float g = gs[tt];
                     if (gate != nullptr && gate_values)      // a gate per value, laid out like the output
-                        g = lat_sigmoid(to_f32(gate[(size_t)t * gate_stride + (size_t)h * dv + i]));
+                        g = sigmoid_f32(to_f32(gate[(size_t)t * gate_stride + (size_t)h * dv + i]));
                     out[(size_t)t * out_stride + (size_t)h * dv + i] = from_f32<T>(acc[tt] * g);
                 }
             }

@@ -18,21 +18,7 @@
 
 #include "lightning.cuh"
 
-__device__ __forceinline__ float light_silu(float x) {
-    float s;
-    if (x >= 0.0f) {
-        s = 1.0f / (1.0f + expf(-x));
-    } else {
-        const float z = expf(x);
-        s = z / (1.0f + z);
-    }
-    return x * s;
-}
-__device__ __forceinline__ float light_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
+__device__ __forceinline__ float light_silu(float x) { return x * sigmoid_f32(x); }
 
 // q and k of one head of the token at row `row` (its q and k heads at qh and kh), activated, rotated and
 // scaled, into shared memory.
@@ -258,7 +244,75 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ x, long x_stride,
     const T* gr = gate + (size_t)t * gate_stride;
     T* yr = y + (size_t)t * y_stride;
     for (int j = threadIdx.x; j < width; j += blockDim.x)
-        yr[j] = from_f32<T>(xr[j] * scale * load_as_f32(w, w_dtype, j) * light_sigmoid(to_f32(gr[j])));
+        yr[j] = from_f32<T>(xr[j] * scale * load_as_f32(w, w_dtype, j) * sigmoid_f32(to_f32(gr[j])));
+}
+
+// The same for rows in whole groups of 4 values, at most 4 * GR_THREADS * 8 of them: a thread keeps its share of the row
+// in registers, asked for with its gates before the norm, so everything is read once and 16 bytes at a time.  Bound by memory: 3,523
+// rows of 4,096 values (bfloat16 gates) 78 -> @@ us with the launch.
+#define GR_THREADS 256
+__device__ __forceinline__ float4 gr_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 gr_load4(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                       __uint_as_float(raw.y & 0xffff0000u));
+}
+__device__ __forceinline__ void gr_store4(float* p, const float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void gr_store4(bf16* p, const float4 v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+template <typename T, int VPL>
+__global__ void __launch_bounds__(GR_THREADS)
+gated_rmsnorm_vec_kernel(const float* __restrict__ x, long x_stride, const T* __restrict__ gate, long gate_stride, const void* __restrict__ w,
+                         int w_dtype, T* __restrict__ y, long y_stride, int width, float eps) {
+    pdl_trigger();
+    __shared__ float scratch[33];
+    const int t = blockIdx.x, n4 = width >> 2;
+    const float* xr = x + (size_t)t * x_stride;
+    const T* gr = gate + (size_t)t * gate_stride;
+    T* yr = y + (size_t)t * y_stride;
+    pdl_wait();
+    float4 v[VPL], g[VPL];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+        const int j = i * GR_THREADS + threadIdx.x;
+        v[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < n4) v[i] = gr_load4(xr + j * 4), g[i] = gr_load4(gr + j * 4);
+    }
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+        ss = fmaf(v[i].x, v[i].x, ss), ss = fmaf(v[i].y, v[i].y, ss), ss = fmaf(v[i].z, v[i].z, ss), ss = fmaf(v[i].w, v[i].w, ss);
+    ss = block_sum(ss, scratch);
+    const float scale = 1.0f / sqrtf(ss / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+        const int j = i * GR_THREADS + threadIdx.x;
+        if (j >= n4) continue;
+        const float4 wv = w_dtype == BFI_F32 ? gr_load4(reinterpret_cast<const float*>(w) + j * 4) : gr_load4(reinterpret_cast<const bf16*>(w) + j * 4);
+        gr_store4(yr + j * 4, make_float4(v[i].x * scale * wv.x * sigmoid_f32(g[i].x), v[i].y * scale * wv.y * sigmoid_f32(g[i].y),
+                                          v[i].z * scale * wv.z * sigmoid_f32(g[i].z), v[i].w * scale * wv.w * sigmoid_f32(g[i].w)));
+    }
+}
+
+template <typename T>
+static bool launch_gated_rmsnorm_vec(const float* x, long x_stride, const T* gate, long gate_stride, const void* w, int w_dtype, T* y, long y_stride,
+                                     int n_rows, int width, float eps, cudaStream_t stream) {
+    const auto al = [](const void* p, size_t n) { return ((uintptr_t)p & (n - 1)) == 0; };
+    if (width % 4 != 0 || width > 4 * GR_THREADS * 8 || x_stride % 4 != 0 || gate_stride % 4 != 0 || y_stride % 4 != 0 || !al(x, 16) ||
+        !al(gate, 4 * sizeof(T)) || !al(y, 4 * sizeof(T)) || !al(w, 4 * (size_t)dtype_size(w_dtype)))
+        return false;
+#define BFI_GR(V)                                                                                                                            \
+    bfi_launch(gated_rmsnorm_vec_kernel<T, V>, dim3(n_rows), dim3(GR_THREADS), 0, stream, x, x_stride, gate, gate_stride, w, w_dtype, y, y_stride, \
+               width, eps)
+    const int per = (width / 4 + GR_THREADS - 1) / GR_THREADS;
+    if (per <= 1) BFI_GR(1);
+    else if (per <= 2) BFI_GR(2);
+    else if (per <= 4) BFI_GR(4);
+    else BFI_GR(8);
+#undef BFI_GR
+    return true;
 }
 
 extern "C" int bfi_gated_rmsnorm(const float* x, long x_stride, const void* gate, long gate_stride, int dtype, const void* w,
@@ -267,6 +321,9 @@ extern "C" int bfi_gated_rmsnorm(const float* x, long x_stride, const void* gate
     BFI_REQUIRE(n_rows >= 0 && width > 0, "gated_rmsnorm: bad sizes rows=%d width=%d", n_rows, width);
     BFI_REQUIRE(x_stride >= width && gate_stride >= width && y_stride >= width, "gated_rmsnorm: row stride shorter than the row");
     if (n_rows == 0) return 0;
+    if (dtype == BFI_F32 ? launch_gated_rmsnorm_vec<float>(x, x_stride, (const float*)gate, gate_stride, w, w_dtype, (float*)y, y_stride, n_rows, width, eps, stream)
+                         : launch_gated_rmsnorm_vec<bf16>(x, x_stride, (const bf16*)gate, gate_stride, w, w_dtype, (bf16*)y, y_stride, n_rows, width, eps, stream))
+        return bfi_check_launch("gated_rmsnorm");
     const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
     if (dtype == BFI_F32)
         bfi_launch(gated_rmsnorm_kernel<float>, dim3(n_rows), dim3(threads), 0, stream, x, x_stride, (const float*)gate, gate_stride, w,

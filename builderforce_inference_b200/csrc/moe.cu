@@ -34,12 +34,6 @@
 // activations per token); its activations are multiplied by the token's gate.
 #include "common.cuh"
 
-__device__ __forceinline__ float moe_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
-
 // The decision of one token, by one warp: zr[0..E) are its logits (zr[E] the extra one), s, choice
 // (E floats each) and gs (n_groups floats) are the warp's scratch in shared memory.
 __device__ __forceinline__ void moe_route_token(const float* zr, const float* __restrict__ correction, int* __restrict__ idx,
@@ -51,7 +45,7 @@ __device__ __forceinline__ void moe_route_token(const float* zr, const float* __
         for (int e = lane; e < E; e += 32) dense_weight[(size_t)t * E + e] = 0.0f;
     if (score_mode == 1) {
         for (int e = lane; e < E; e += 32) {
-            s[e] = moe_sigmoid(zr[e]);
+            s[e] = sigmoid_f32(zr[e]);
             choice[e] = s[e] + (correction ? correction[e] : 0.0f);
         }
     } else {
@@ -142,7 +136,7 @@ __device__ __forceinline__ void moe_route_token(const float* zr, const float* __
         }
         __syncwarp();
     }
-    if (extra && lane == 0) gate[t] = moe_sigmoid(zr[E]);
+    if (extra && lane == 0) gate[t] = sigmoid_f32(zr[E]);
 }
 
 // One warp per token, logits given.  Shared memory per warp: s[E], choice[E], group[n_groups].

@@ -23,12 +23,7 @@
 #define REC_DECAY_SIGMOID 2
 #define REC_MAX_TAPS 16
 
-__device__ __forceinline__ float rec_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
-__device__ __forceinline__ float rec_silu(float x) { return x * rec_sigmoid(x); }
+__device__ __forceinline__ float rec_silu(float x) { return x * sigmoid_f32(x); }
 __device__ __forceinline__ float rec_softplus(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
 __device__ __forceinline__ float rec_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
 
@@ -937,7 +932,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ x, long x_stri
             float v = xr[j0 + j];
             if (gate_first) {
                 const float gv = to_f32(gr[j0 + j]);
-                v *= gate_act ? rec_silu(gv) : rec_sigmoid(gv);
+                v *= gate_act ? rec_silu(gv) : sigmoid_f32(gv);
             }
             ss = fmaf(v, v, ss);
         }
@@ -945,7 +940,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ x, long x_stri
         const float scale = 1.0f / sqrtf(ss / (float)len + eps);
         for (int j = lane; j < len; j += 32) {
             const float gv = to_f32(gr[j0 + j]);
-            const float ga = gate_act ? rec_silu(gv) : rec_sigmoid(gv);
+            const float ga = gate_act ? rec_silu(gv) : sigmoid_f32(gv);
             yr[j0 + j] = from_f32<T>(xr[j0 + j] * ga * scale * (w != nullptr ? load_as_f32(w, w_dtype, (j0 + j) % w_len) : 1.0f));
         }
     }
@@ -995,7 +990,7 @@ gated_group_norm_vec_kernel(const float* __restrict__ x, long x_stride, const T*
     for (int i = 0; i < VPL; ++i) {
         float4& a = g[i];
         if (gate_act) a = make_float4(rec_silu(a.x), rec_silu(a.y), rec_silu(a.z), rec_silu(a.w));
-        else a = make_float4(rec_sigmoid(a.x), rec_sigmoid(a.y), rec_sigmoid(a.z), rec_sigmoid(a.w));
+        else a = make_float4(sigmoid_f32(a.x), sigmoid_f32(a.y), sigmoid_f32(a.z), sigmoid_f32(a.w));
         if (gate_first) {
             const float4 u = make_float4(v[i].x * a.x, v[i].y * a.y, v[i].z * a.z, v[i].w * a.w);
             ss = fmaf(u.x, u.x, ss), ss = fmaf(u.y, u.y, ss), ss = fmaf(u.z, u.z, ss), ss = fmaf(u.w, u.w, ss);

@@ -24,12 +24,6 @@ struct NormAddGate {
     int bias_dtype;
 };
 
-__device__ __forceinline__ float out_sigmoid(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float z = expf(x);
-    return z / (1.0f + z);
-}
-
 __global__ void norm_add_kernel(float* __restrict__ x, long x_stride, const float* __restrict__ y, long y_stride,
                                 const void* __restrict__ w, int w_dtype, int width, float eps, const void* __restrict__ w2,
                                 int w2_dtype, float eps2, void* __restrict__ h, int h_dtype, long h_stride, float mult,
@@ -47,7 +41,7 @@ __global__ void norm_add_kernel(float* __restrict__ x, long x_stride, const floa
         if (gated) {
             float z = load_as_f32(g.logits, g.dtype, (size_t)t * g.stride + j);
             if (g.bias) z += load_as_f32(g.bias, g.bias_dtype, j);
-            v *= out_sigmoid(z);
+            v *= sigmoid_f32(z);
         }
         ss = fmaf(v, v, ss);
     }
@@ -59,7 +53,7 @@ __global__ void norm_add_kernel(float* __restrict__ x, long x_stride, const floa
         if (gated) {
             float z = load_as_f32(g.logits, g.dtype, (size_t)t * g.stride + j);
             if (g.bias) z += load_as_f32(g.bias, g.bias_dtype, j);
-            yv *= out_sigmoid(z);
+            yv *= sigmoid_f32(z);
         }
         const float v = xr[j] + mult * (yv * scale * load_as_f32(w, w_dtype, j));
         xr[j] = v;
@@ -186,10 +180,10 @@ norm_add_vec_kernel(float* __restrict__ x, long x_stride, const float* __restric
                 const float4 b = load4_as_f32(g.bias, g.bias_dtype, (size_t)j * 4);
                 z.x += b.x, z.y += b.y, z.z += b.z, z.w += b.w;
             }
-            v[i].x *= out_sigmoid(z.x);
-            v[i].y *= out_sigmoid(z.y);
-            v[i].z *= out_sigmoid(z.z);
-            v[i].w *= out_sigmoid(z.w);
+            v[i].x *= sigmoid_f32(z.x);
+            v[i].y *= sigmoid_f32(z.y);
+            v[i].z *= sigmoid_f32(z.z);
+            v[i].w *= sigmoid_f32(z.w);
         }
         ss = fmaf(v[i].x, v[i].x, ss);
         ss = fmaf(v[i].y, v[i].y, ss);

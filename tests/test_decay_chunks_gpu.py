@@ -97,3 +97,17 @@ def test_decays_that_leave_nothing_and_values_that_are_not_finite(mode):
     same = torch.isfinite(plain)
     assert torch.equal(torch.isfinite(out), same) and torch.equal(torch.isfinite(S_out), torch.isfinite(S_plain))
     assert bool(same[:100].all()) and err(out[same], plain[same].to(F64)) < 2e-6
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [4, 1000, 1028, 2048, 4096, 8192, 8196])
+def test_gated_norm_of_rows_in_whole_groups(dt, width):
+    """Rows kept in registers, one to eight groups of four values a thread; one group more takes the general kernel."""
+    from builderforce_inference_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(width)
+    x, w = torch.randn(3, width, generator=g, device=DEV), 1 + 0.1 * torch.randn(width, generator=g, device=DEV)
+    gate = (40.0 * torch.randn(3, width + 8, generator=g, device=DEV)).to(dt)[:, 8:]
+    out = torch.empty(3, width, dtype=dt, device=DEV)
+    ops.gated_rmsnorm(x, gate, w, 1e-5, out)
+    ref = x.to(F64) * torch.rsqrt(x.to(F64).square().mean(1, keepdim=True) + 1e-5) * w.to(F64) * torch.sigmoid(gate.to(F64))
+    assert err(out, ref) < (5e-7 if dt == torch.float32 else 2.0 ** -8)
