@@ -249,7 +249,7 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ x, long x_stride,
 
 // The same for rows in whole groups of 4 values, at most 4 * GR_THREADS * 8 of them: a thread keeps its share of the row
 // in registers, asked for with its gates before the norm, so everything is read once and 16 bytes at a time.  Bound by memory: 3,523
-// rows of 4,096 values (bfloat16 gates) 78 -> @@ us with the launch.
+// rows of 4,096 values (bfloat16 gates) took 78 us twice over the row, four bytes at a time and both branches of the sigmoid; 38 now.
 #define GR_THREADS 256
 __device__ __forceinline__ float4 gr_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 gr_load4(const bf16* p) {
