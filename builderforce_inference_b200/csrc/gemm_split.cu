@@ -26,12 +26,13 @@
 // other's shared memory.
 //
 // What bounds it: the tensor pipe (six bfloat16 products for one of float32, 1657 / 6 = 276 TFLOP/s of the
-// measured peak); a block of 32 k takes 1.84 us at 256 features, 12 instructions of 0.12 us and what the workers'
-// shared-memory traffic adds.  The float32 multiply-adds of 148 x 128 lanes are 74 TFLOP/s; gemm_simt.cu reaches 25.
+// measured peak) and, before that, the splitting: a block of 32 k at 256 features takes 1.77 us, where the 12 products alone
+// take 0.91 and the workers alone 1.52 (0.0028 us a row of A or W and 0.35 for the barriers and the fence).
+// The float32 multiply-adds of 148 x 128 lanes are 74 TFLOP/s; gemm_simt.cu reaches 25.
 // Tokens x features x k, gemm_simt.cu -> this kernel:
-//     1134 x 6144 x 2560    1435 -> 269 us (133 TFLOP/s)      1134 x 2560 x 9728    2749 -> 408 us (138 TFLOP/s)
-//      333 x 2560 x 4096     648 ->  69 us                      64 x 19456 x 2560    515 -> 130 us
-//       24 x 6144 x 2560     183 ->  37 us                      40 x 2560 x 2560     181 ->  23 us
+//     1134 x 6144 x 2560    1435 -> 256 us (140 TFLOP/s)      1134 x 2560 x 9728    2749 -> 403 us (140 TFLOP/s)
+//      333 x 2560 x 4096     648 ->  69 us                      64 x 19456 x 2560    515 -> 124 us
+//       24 x 6144 x 2560     183 ->  37 us                      40 x 2560 x 2560     181 ->  24 us
 //
 // Every wait on an mbarrier is bounded: one that runs out records BFI_STATUS_TIMEOUT and the block returns.
 #include "tcgen05.cuh"
@@ -70,6 +71,9 @@ __device__ __forceinline__ void gs_meet(int ksplit) {
         asm volatile("bar.sync 0, %0;" ::"n"(GS_THREADS) : "memory");
 }
 
+// TW: tasks of 64 rows of W a worker has (the tile's width in 64s, rounded up): a constant, so that a block's tasks are straight-line
+// code whose chains of conversions run side by side.
+template <int TW>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, void* __restrict__ C, int c_dtype,
                   long ldc, int M, int N, int K, int tile_n, int kblocks_per_split, int epilogue, int vec_ok, GateAct gate,
@@ -116,19 +120,19 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
         const int t = threadIdx.x, r0 = t >> 2, ch = t & 3;
         const float* a_ptr = A + (size_t)min(m0 + r0, M - 1) * lda + ch * 8;
         const float* a_ptr1 = A + (size_t)min(m0 + r0 + 64, M - 1) * lda + ch * 8;
-        const float* w_ptr[4];
+        const float* w_ptr[TW];
         uint32_t live = (m0 + r0 < M ? 1u : 0u) | (m0 + r0 + 64 < M ? 2u : 0u);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < TW; ++j) {
             const int r = r0 + 64 * j;
             w_ptr[j] = W + (size_t)min(n0 + r, N - 1) * ldw + ch * 8;
             if (r < tile_n && n0 + r < N) live |= 4u << j;
         }
         const uint32_t at = (uint32_t)r0 * 64 + (uint32_t)((ch ^ ((r0 >> 1) & 3)) << 4);       // rows 64 on share it: 64 rows are whole swizzle groups
-        float4 x[6][2];
+        float4 x[2 + TW][2];
         auto fetch = [&](int j, int kb) {                  // j a constant: x stays in registers
             const int k = kb * GS_BK;
-            const float* p = (j == 0 ? a_ptr : j == 1 ? a_ptr1 : w_ptr[(j + 2) & 3]) + k;
+            const float* p = (j == 0 ? a_ptr : j == 1 ? a_ptr1 : w_ptr[j < 2 ? 0 : j - 2]) + k;
             const bool on = (live >> j) & 1;
             x[j][0] = on && k + ch * 8 < K ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
             x[j][1] = on && k + ch * 8 + 4 < K ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -159,7 +163,7 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
         bool ok = true;
         int chains = 0;                                    // fetched so far
 #pragma unroll
-        for (int j = 0; j < 6; ++j) fetch(j, kb_beg);
+        for (int j = 0; j < 2 + TW; ++j) fetch(j, kb_beg);
         for (int i = 0; i < n_kb; ++i) {
             const int s = i % GS_STAGES;
             if (i >= GS_STAGES && !MBAR_WAIT(&empty[s], ((uint32_t)(i / GS_STAGES) & 1) ^ 1)) {
@@ -179,14 +183,13 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
             }
             unsigned char* stage = smem + (size_t)s * GS_STAGE_BYTES;
 #pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                if (j >= 2 && (j - 2) * 64 >= tile_n) break;
+            for (int j = 0; j < 2 + TW; ++j) {
                 uint4 h, m, l;
                 split_pair(x[j][0].x, x[j][0].y, h.x, m.x, l.x);
                 split_pair(x[j][0].z, x[j][0].w, h.y, m.y, l.y);
                 split_pair(x[j][1].x, x[j][1].y, h.z, m.z, l.z);
                 split_pair(x[j][1].z, x[j][1].w, h.w, m.w, l.w);
-                if (i + 1 < n_kb) fetch(j, kb_beg + i + 1);            // travels while the other tasks are split
+                fetch(j, kb_beg + i + 1);                              // travels while the other tasks are split (past K: zeros; past the split: not used)
                 unsigned char* dst = stage + at + (j < 2 ? j * 64 * 64 : 3 * GS_A_TERM + (j - 2) * 64 * 64);
                 const uint32_t term = j < 2 ? GS_A_TERM : GS_W_TERM;
                 *reinterpret_cast<uint4*>(dst) = h;
@@ -355,10 +358,11 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
 
 // Reserves the kernel's shared memory; how many clusters of 2 to 8 blocks the GPU holds at once (a cluster lives
 // in one group of SMs, so these are fewer than the SMs divided by its size).  Null after recording an error.
+template <int TW>
 static const int* gs_clusters() {
     static int most[9];
     static const bool ok = [] {
-        cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GS_SMEM);
         for (int ks = 2; ks <= 8 && e == cudaSuccess; ++ks) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
@@ -371,7 +375,7 @@ static const int* gs_clusters() {
             cfg.dynamicSmemBytes = GS_SMEM;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            e = cudaOccupancyMaxActiveClusters(&most[ks], gemm_split_kernel, &cfg);
+            e = cudaOccupancyMaxActiveClusters(&most[ks], gemm_split_kernel<TW>, &cfg);
         }
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -408,8 +412,8 @@ extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long
     // the tile's width and the splits of K that take the least time by an estimate: rounds over the SMs x (blocks
     // of k x 12 products, which take nearly as long for 128 features as for 256, + what surrounds them)
     const int kb = (K + GS_BK - 1) / GS_BK, n_sm = bfi_sm_count();
-    const int* clusters = gs_clusters();
-    if (clusters == nullptr) return 1;
+    const int* clusters = gs_clusters<4>();
+    if (clusters == nullptr || gs_clusters<1>() == nullptr || gs_clusters<2>() == nullptr || gs_clusters<3>() == nullptr) return 1;
     int tile_n = GS_FEATS, ksplit = 1;
     double best = -1.0;
     for (int ks = 1; ks <= 8; ++ks) {
@@ -427,6 +431,7 @@ extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long
     const int per_split = (kb + ksplit - 1) / ksplit;
     ksplit = (kb + per_split - 1) / per_split;             // no empty splits
 
+    auto kernel = tile_n <= 64 ? gemm_split_kernel<1> : tile_n <= 128 ? gemm_split_kernel<2> : tile_n <= 192 ? gemm_split_kernel<3> : gemm_split_kernel<4>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((N + tile_n - 1) / tile_n, tiles_m, ksplit);
     cfg.blockDim = dim3(GS_THREADS);
@@ -449,7 +454,7 @@ extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     const int vec_ok = (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel, A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split, epilogue, vec_ok,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split, epilogue, vec_ok,
                                        g_bfi_gate, status);
     if (e != cudaSuccess) {
         cudaGetLastError();
