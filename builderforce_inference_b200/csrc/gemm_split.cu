@@ -26,13 +26,13 @@
 // other's shared memory.
 //
 // What bounds it: the tensor pipe (six bfloat16 products for one of float32, 1657 / 6 = 276 TFLOP/s of the
-// measured peak) and, before that, the splitting: a block of 32 k at 256 features takes 1.77 us, where the 12 products alone
-// take 0.91 and the workers alone 1.52 (0.0028 us a row of A or W and 0.35 for the barriers and the fence).
+// measured peak) and, before that, the workers: a block of 32 k at 256 features takes 1.73 to 1.76 us; 1.54 without the products,
+// 0.92 with nothing but the products, 1.21 without the loads.
 // The float32 multiply-adds of 148 x 128 lanes are 74 TFLOP/s; gemm_simt.cu reaches 25.
 // Tokens x features x k, gemm_simt.cu -> this kernel:
-//     1134 x 6144 x 2560    1435 -> 256 us (140 TFLOP/s)      1134 x 2560 x 9728    2749 -> 403 us (140 TFLOP/s)
-//      333 x 2560 x 4096     648 ->  69 us                      64 x 19456 x 2560    515 -> 124 us
-//       24 x 6144 x 2560     183 ->  37 us                      40 x 2560 x 2560     181 ->  24 us
+//     1134 x 6144 x 2560    1435 -> 262 us (136 TFLOP/s)      1134 x 2560 x 9728    2749 -> 405 to 445 us
+//      333 x 2560 x 4096     648 ->  67 us                      64 x 19456 x 2560    515 -> 125 us
+//       24 x 6144 x 2560     183 ->  37 us                      40 x 2560 x 2560     181 ->  22 us
 //
 // Every wait on an mbarrier is bounded: one that runs out records BFI_STATUS_TIMEOUT and the block returns.
 #include "tcgen05.cuh"
@@ -72,7 +72,7 @@ __device__ __forceinline__ void gs_meet(int ksplit) {
 }
 
 // TW: tasks of 64 rows of W a worker has (the tile's width in 64s, rounded up): a constant, so that a block's tasks are straight-line
-// code whose chains of conversions run side by side.
+// code (1134 x 19456 x 2560: 829 -> 814 us; 40 x 2560 x 2560: 22.9 -> 21.9).
 template <int TW>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, void* __restrict__ C, int c_dtype,
@@ -189,7 +189,7 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
                 split_pair(x[j][0].z, x[j][0].w, h.y, m.y, l.y);
                 split_pair(x[j][1].x, x[j][1].y, h.z, m.z, l.z);
                 split_pair(x[j][1].z, x[j][1].w, h.w, m.w, l.w);
-                fetch(j, kb_beg + i + 1);                              // travels while the other tasks are split (past K: zeros; past the split: not used)
+                if (i + 1 < n_kb) fetch(j, kb_beg + i + 1);            // travels while the other tasks are split (always fetching costs short splits up to 8%)
                 unsigned char* dst = stage + at + (j < 2 ? j * 64 * 64 : 3 * GS_A_TERM + (j - 2) * 64 * 64);
                 const uint32_t term = j < 2 ? GS_A_TERM : GS_W_TERM;
                 *reinterpret_cast<uint4*>(dst) = h;
