@@ -25,6 +25,13 @@
 // With K split, the blocks of a tile form a cluster and add their partial tiles in split order out of each
 // other's shared memory.
 //
+// With more than one tile of tokens a row of W would be split once a tile.  Where two estimates (gs_tile, gs_plan) say that it
+// pays, split_terms_kernel writes both operands' terms to scratch first, as the ring holds them, and the blocks only copy:
+// tokens x features x k, split in the product -> ahead, with the splitting:
+//     1134 x 6144 x 2560     265 -> 192 us      1134 x 19456 x 2560    879 -> 583 us      1134 x 2560 x 4096    196 -> 141 us
+//      512 x 6144 x 2560     137 -> 102 us       900 x 1536 x 1000      35 ->  31 us      4096 x 6144 x 2560    967 -> 597 us
+//      512 x 512 x 512        16 ->  23 us, 256 x 2560 x 4096    59 ->  61 us, 129 x 40000 x 768    143 -> 151 us: not taken
+//
 // What bounds it: the tensor pipe (six bfloat16 products for one of float32, 1657 / 6 = 276 TFLOP/s of the
 // measured peak) and, before that, the workers: a block of 32 k at 256 features takes 1.73 to 1.76 us; 1.54 without the products,
 // 0.92 with nothing but the products, 1.21 without the loads.
@@ -46,6 +53,9 @@
 #define GS_BK 32                                      // k values per block: 64 bytes of a term
 #define GS_CHAIN 4                                    // blocks of k between two fetches of the h h chain
 #define GS_STAGES 3
+#define GS_TERMS_A (96L << 20)                         // most bytes of A's and of W's terms at a time
+#define GS_TERMS_W (160L << 20)
+#define GS_TERMS_L2 (96L << 20)                        // terms that are still in the L2 when the product reads them
 #define GS_MIN_K 512                                  // shorter sums: the multiply-adds' own rounding can be as small as the truncation of a chain
 #define GS_WORKERS 8
 #define GS_THREADS (GS_WORKERS * 32 + 128)             // a worker holds 128 sums: the registers are split 232 / 40 between the warpgroups
@@ -71,13 +81,66 @@ __device__ __forceinline__ void gs_meet(int ksplit) {
         asm volatile("bar.sync 0, %0;" ::"n"(GS_THREADS) : "memory");
 }
 
+// Both operands' terms, split ahead of the product (split_terms_kernel), and the tile the launch begins with.  Per block of 32 k
+// and per term there are `rows` rows of 64 bytes, swizzled as the ring holds them: a tile's share is one contiguous copy.
+struct GsTerms {
+    const unsigned char *a, *w;
+    int a_rows, w_rows;
+    int tile_x, tile_y;
+};
+struct GsOperand {
+    const float* x;
+    long ld;
+    int first, rows, live;                                 // rows `first` on of x; `rows` written, those from `live` on (of all of x) as zeros
+    unsigned char* out;
+};
+
+// The terms of a piece of A and of a piece of W.  Bound by memory (4 bytes read, 6 written a value): 64 rows x 4 blocks of k per
+// block of threads, four lanes to a row's 128 bytes, and a thread's eight loads in flight before the first is split.
+__global__ void __launch_bounds__(256) split_terms_kernel(GsOperand a, GsOperand w, int a_blocks, int K) {
+    pdl_trigger();
+    pdl_wait();
+    const GsOperand o = (int)blockIdx.x < a_blocks ? a : w;
+    const int r = ((int)blockIdx.x - ((int)blockIdx.x < a_blocks ? 0 : a_blocks)) * 64 + (threadIdx.x >> 2), ch = threadIdx.x & 3;
+    const int n_kb = (K + GS_BK - 1) / GS_BK;
+    if (r >= o.rows) return;
+    const bool on = o.first + r < o.live;
+    const float* p = o.x + (size_t)(on ? o.first + r : 0) * o.ld;
+    float4 x[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int k = ((int)blockIdx.y * 4 + u) * GS_BK + ch * 8;
+        x[u][0] = on && k < K ? *reinterpret_cast<const float4*>(p + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[u][1] = on && k + 4 < K ? *reinterpret_cast<const float4*>(p + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int kb = (int)blockIdx.y * 4 + u;
+        if (kb >= n_kb) return;
+        uint4 t[3];
+        split_pair(x[u][0].x, x[u][0].y, t[0].x, t[1].x, t[2].x);
+        split_pair(x[u][0].z, x[u][0].w, t[0].y, t[1].y, t[2].y);
+        split_pair(x[u][1].x, x[u][1].y, t[0].z, t[1].z, t[2].z);
+        split_pair(x[u][1].z, x[u][1].w, t[0].w, t[1].w, t[2].w);
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            *reinterpret_cast<uint4*>(o.out + ((size_t)(kb * 3 + j) * o.rows + r) * 64 + ((ch ^ ((r >> 1) & 3)) << 4)) = t[j];
+    }
+}
+
+// `bytes` and both addresses are multiples of 16.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
 // TW: tasks of 64 rows of W a worker has (the tile's width in 64s, rounded up): a constant, so that a block's tasks are straight-line
-// code (1134 x 19456 x 2560: 829 -> 814 us; 40 x 2560 x 2560: 22.9 -> 21.9).
+// code (1134 x 19456 x 2560: 829 -> 814 us; 40 x 2560 x 2560: 22.9 -> 21.9).  TW = 0: the operands come as terms, one lane of warp 9 copies them into the ring and the workers only keep the sums.
 template <int TW>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, void* __restrict__ C, int c_dtype,
                   long ldc, int M, int N, int K, int tile_n, int kblocks_per_split, int epilogue, int vec_ok, GateAct gate,
-                  int* __restrict__ status) {
+                  GsTerms terms, int* __restrict__ status) {
     const uint32_t spin_limit = TC_SPIN_LIMIT;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -88,7 +151,7 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(chain_empty + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * GS_TOKENS, n0 = blockIdx.x * tile_n;
+    const int m0 = (terms.tile_y + (int)blockIdx.y) * GS_TOKENS, n0 = (terms.tile_x + (int)blockIdx.x) * tile_n;
     const int ksplit = gridDim.z;
     const int all_kb = (K + GS_BK - 1) / GS_BK;
     const int kb_beg = blockIdx.z * kblocks_per_split;
@@ -96,7 +159,7 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < GS_STAGES; ++s) {
-            mbar_init(&full[s], GS_WORKERS);
+            mbar_init(&full[s], TW > 0 ? GS_WORKERS : 1);
             mbar_init(&empty[s], 1);
         }
         mbar_init(chain_full, 1);
@@ -117,27 +180,6 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
     if (warp < GS_WORKERS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");      // 256 x 232 + 128 x 40 = 384 x 168, what the block was launched with
         // ---------------- workers.  Task j of a thread: 8 values of k of one row; j 0, 1: A, 2..5: W
-        const int t = threadIdx.x, r0 = t >> 2, ch = t & 3;
-        const float* a_ptr = A + (size_t)min(m0 + r0, M - 1) * lda + ch * 8;
-        const float* a_ptr1 = A + (size_t)min(m0 + r0 + 64, M - 1) * lda + ch * 8;
-        const float* w_ptr[TW];
-        uint32_t live = (m0 + r0 < M ? 1u : 0u) | (m0 + r0 + 64 < M ? 2u : 0u);
-#pragma unroll
-        for (int j = 0; j < TW; ++j) {
-            const int r = r0 + 64 * j;
-            w_ptr[j] = W + (size_t)min(n0 + r, N - 1) * ldw + ch * 8;
-            if (r < tile_n && n0 + r < N) live |= 4u << j;
-        }
-        const uint32_t at = (uint32_t)r0 * 64 + (uint32_t)((ch ^ ((r0 >> 1) & 3)) << 4);       // rows 64 on share it: 64 rows are whole swizzle groups
-        float4 x[2 + TW][2];
-        auto fetch = [&](int j, int kb) {                  // j a constant: x stays in registers
-            const int k = kb * GS_BK;
-            const float* p = (j == 0 ? a_ptr : j == 1 ? a_ptr1 : w_ptr[j < 2 ? 0 : j - 2]) + k;
-            const bool on = (live >> j) & 1;
-            x[j][0] = on && k + ch * 8 < K ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-            x[j][1] = on && k + ch * 8 + 4 < K ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        };
-
         const int quad = warp & 3;
         const int pairs = (tile_n / 16 + 1) / 2, first_pair = warp < 4 ? 0 : (pairs + 1) / 2;
         const int my_pairs = warp < 4 ? (pairs + 1) / 2 : pairs - first_pair;                  // of 32 features, at most 4
@@ -162,43 +204,65 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
 
         bool ok = true;
         int chains = 0;                                    // fetched so far
+        if constexpr (TW > 0) {
+            const int t = threadIdx.x, r0 = t >> 2, ch = t & 3;
+            const float* a_ptr = A + (size_t)min(m0 + r0, M - 1) * lda + ch * 8;
+            const float* a_ptr1 = A + (size_t)min(m0 + r0 + 64, M - 1) * lda + ch * 8;
+            const float* w_ptr[TW];
+            uint32_t live = (m0 + r0 < M ? 1u : 0u) | (m0 + r0 + 64 < M ? 2u : 0u);
 #pragma unroll
-        for (int j = 0; j < 2 + TW; ++j) fetch(j, kb_beg);
-        for (int i = 0; i < n_kb; ++i) {
-            const int s = i % GS_STAGES;
-            if (i >= GS_STAGES && !MBAR_WAIT(&empty[s], ((uint32_t)(i / GS_STAGES) & 1) ^ 1)) {
-                ok = false;
-                break;
+            for (int j = 0; j < TW; ++j) {
+                const int r = r0 + 64 * j;
+                w_ptr[j] = W + (size_t)min(n0 + r, N - 1) * ldw + ch * 8;
+                if (r < tile_n && n0 + r < N) live |= 4u << j;
             }
-            if (i >= GS_CHAIN + 2 && i % GS_CHAIN == 2) {
-                // block i - 3, the chain's last, is done: this wait returns at once
-                if (!MBAR_WAIT(chain_full, (uint32_t)chains & 1)) {
+            const uint32_t at = (uint32_t)r0 * 64 + (uint32_t)((ch ^ ((r0 >> 1) & 3)) << 4);       // rows 64 on share it: 64 rows are whole swizzle groups
+            float4 x[2 + TW][2];
+            auto fetch = [&](int j, int kb) {                  // j a constant: x stays in registers
+                const int k = kb * GS_BK;
+                const float* p = (j == 0 ? a_ptr : j == 1 ? a_ptr1 : w_ptr[j < 2 ? 0 : j - 2]) + k;
+                const bool on = (live >> j) & 1;
+                x[j][0] = on && k + ch * 8 < K ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[j][1] = on && k + ch * 8 + 4 < K ? *reinterpret_cast<const float4*>(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+#pragma unroll
+            for (int j = 0; j < 2 + TW; ++j) fetch(j, kb_beg);
+            for (int i = 0; i < n_kb; ++i) {
+                const int s = i % GS_STAGES;
+                if (i >= GS_STAGES && !MBAR_WAIT(&empty[s], ((uint32_t)(i / GS_STAGES) & 1) ^ 1)) {
                     ok = false;
                     break;
                 }
-                add_chain(lane_addr);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(chain_empty);
-                ++chains;
-            }
-            unsigned char* stage = smem + (size_t)s * GS_STAGE_BYTES;
+                if (i >= GS_CHAIN + 2 && i % GS_CHAIN == 2) {
+                    // block i - 3, the chain's last, is done: this wait returns at once
+                    if (!MBAR_WAIT(chain_full, (uint32_t)chains & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    add_chain(lane_addr);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(chain_empty);
+                    ++chains;
+                }
+                unsigned char* stage = smem + (size_t)s * GS_STAGE_BYTES;
 #pragma unroll
-            for (int j = 0; j < 2 + TW; ++j) {
-                uint4 h, m, l;
-                split_pair(x[j][0].x, x[j][0].y, h.x, m.x, l.x);
-                split_pair(x[j][0].z, x[j][0].w, h.y, m.y, l.y);
-                split_pair(x[j][1].x, x[j][1].y, h.z, m.z, l.z);
-                split_pair(x[j][1].z, x[j][1].w, h.w, m.w, l.w);
-                if (i + 1 < n_kb) fetch(j, kb_beg + i + 1);            // travels while the other tasks are split (always fetching costs short splits up to 8%)
-                unsigned char* dst = stage + at + (j < 2 ? j * 64 * 64 : 3 * GS_A_TERM + (j - 2) * 64 * 64);
-                const uint32_t term = j < 2 ? GS_A_TERM : GS_W_TERM;
-                *reinterpret_cast<uint4*>(dst) = h;
-                *reinterpret_cast<uint4*>(dst + term) = m;
-                *reinterpret_cast<uint4*>(dst + 2 * term) = l;
+                for (int j = 0; j < 2 + TW; ++j) {
+                    uint4 h, m, l;
+                    split_pair(x[j][0].x, x[j][0].y, h.x, m.x, l.x);
+                    split_pair(x[j][0].z, x[j][0].w, h.y, m.y, l.y);
+                    split_pair(x[j][1].x, x[j][1].y, h.z, m.z, l.z);
+                    split_pair(x[j][1].z, x[j][1].w, h.w, m.w, l.w);
+                    if (i + 1 < n_kb) fetch(j, kb_beg + i + 1);            // travels while the other tasks are split (always fetching costs short splits up to 8%)
+                    unsigned char* dst = stage + at + (j < 2 ? j * 64 * 64 : 3 * GS_A_TERM + (j - 2) * 64 * 64);
+                    const uint32_t term = j < 2 ? GS_A_TERM : GS_W_TERM;
+                    *reinterpret_cast<uint4*>(dst) = h;
+                    *reinterpret_cast<uint4*>(dst + term) = m;
+                    *reinterpret_cast<uint4*>(dst + 2 * term) = l;
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[s]);
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);
         }
         const int all_chains = (n_kb + GS_CHAIN - 1) / GS_CHAIN;
         for (; ok && chains < all_chains; ++chains) {
@@ -343,6 +407,29 @@ gemm_split_kernel(const float* __restrict__ A, long lda, const float* __restrict
             }
             if (!ok) atomicOr(status, BFI_STATUS_TIMEOUT);
         }
+        if (TW == 0 && warp == GS_WORKERS + 1 && lane == 0) {
+            // ---------------- the copies
+            const uint32_t w_bytes = (uint32_t)tile_n * 64;
+            const unsigned char* a = terms.a + (size_t)blockIdx.y * GS_TOKENS * 64;
+            const unsigned char* w = terms.w + (size_t)blockIdx.x * tile_n * 64;
+            int i = 0;
+            for (; i < n_kb; ++i) {
+                const int s = i % GS_STAGES;
+                if (i >= GS_STAGES && !MBAR_WAIT(&empty[s], ((uint32_t)(i / GS_STAGES) & 1) ^ 1)) break;
+                unsigned char* stage = smem + (size_t)s * GS_STAGE_BYTES;
+                mbar_expect_tx(&full[s], 3 * (GS_A_TERM + w_bytes));
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    const size_t at = (size_t)(kb_beg + i) * 3 + t;
+                    bulk_load(stage + t * GS_A_TERM, a + at * terms.a_rows * 64, GS_A_TERM, &full[s]);
+                    bulk_load(stage + 3 * GS_A_TERM + t * GS_W_TERM, w + at * terms.w_rows * 64, w_bytes, &full[s]);
+                }
+            }
+            if (i < n_kb) {
+                atomicOr(status, BFI_STATUS_TIMEOUT);
+                for (int j = max(0, i - GS_STAGES); j < i; ++j) (void)MBAR_WAIT(&full[j % GS_STAGES], (uint32_t)(j / GS_STAGES) & 1);
+            }
+        }
         __syncwarp();
         gs_meet(ksplit);
         gs_meet(ksplit);
@@ -386,12 +473,165 @@ static const int* gs_clusters() {
     return ok ? most : nullptr;
 }
 
+static int gs_launch(decltype(&gemm_split_kernel<0>) kernel, dim3 grid, const float* A, long lda, const float* W, long ldw, void* C, int c_dtype,
+                     long ldc, int M, int N, int K, int tile_n, int per_split, int epilogue, GsTerms terms, int* status, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(GS_THREADS);
+    cfg.dynamicSmemBytes = GS_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (grid.z > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = 1;
+        attr[n_attr].val.clusterDim.y = 1;
+        attr[n_attr].val.clusterDim.z = grid.z;
+        ++n_attr;
+    }
+    if (g_bfi_pdl) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    const int vec_ok = (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split, epilogue, vec_ok,
+                                       g_bfi_gate, terms, status);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return bfi_fail("gemm_split: launch failed: %s", cudaGetErrorString(e));
+    }
+    return bfi_check_launch("gemm_split");
+}
+
+// The tile's width and the splits of K with which splitting as it goes takes the least time by an estimate, which is returned
+// in us: rounds over the SMs x (blocks of k x 12 products and the workers' conversions + what surrounds them).  -1: there is
+// none; -2 after recording an error.
+static double gs_tile(int M, int N, int K, int tune_n, int tune_split, int* tile_n, int* ksplit) {
+    const int kb = (K + GS_BK - 1) / GS_BK, n_sm = bfi_sm_count(), tiles_m = (M + GS_TOKENS - 1) / GS_TOKENS;
+    const int* clusters = gs_clusters<4>();
+    if (clusters == nullptr || gs_clusters<1>() == nullptr || gs_clusters<2>() == nullptr || gs_clusters<3>() == nullptr) return -2.0;
+    double best = -1.0;
+    for (int ks = 1; ks <= 8; ++ks) {
+        if (tune_split > 0 ? ks != tune_split : (ks > 1 && kb / ks < 2 * GS_CHAIN)) continue;
+        for (int tn = GS_FEATS; tn >= 64; tn -= 16) {
+            if (tune_n > 0 && tn != tune_n) continue;
+            const long blocks = (long)tiles_m * ((N + tn - 1) / tn) * ks;
+            const long slots = ks == 1 ? n_sm : (long)clusters[ks] * ks;
+            if (slots < ks) continue;
+            const double cost = (double)((blocks + slots - 1) / slots) * ((double)((kb + ks - 1) / ks) * (1.10 + 0.0026 * tn) + (ks > 1 ? 8.5 : 2.5));
+            if (best < 0.0 || cost < best) best = cost, *tile_n = tn, *ksplit = ks;
+        }
+    }
+    return best;
+}
+
+// How a product runs on operands split ahead: pieces of `m_tiles` x 128 tokens and `n_tiles` x `tile_n` features, whose terms
+// take at most GS_TERMS_A and GS_TERMS_W bytes, so that the scratch stays bounded.  Returns the least time by an estimate in us
+// (negative: there is no plan).  Measured, us, best tile for pieces of 64 MB / of 160: 1134 x 19456 x 2560 557 / 613 (the smaller
+// pieces' terms are read back out of the L2), 1134 x 2560 x 9728 341 / 292 (one piece instead of three).
+struct GsPlan {
+    int tile_n, ksplit, m_tiles, n_tiles;
+    long bytes;
+};
+static double gs_plan(int M, int N, int K, int tune_n, int tune_split, GsPlan* plan) {
+    const int kb = (K + GS_BK - 1) / GS_BK, n_sm = bfi_sm_count();
+    const int* clusters = gs_clusters<0>();
+    if (clusters == nullptr) return -2.0;
+    const long row = (long)kb * 3 * 64;
+    const int tiles_m = (M + GS_TOKENS - 1) / GS_TOKENS;
+    const long most_m = GS_TERMS_A / (row * GS_TOKENS);
+    if (most_m < 1) return -1.0;
+    const int m_pieces = (int)((tiles_m + most_m - 1) / most_m);
+    plan->m_tiles = (tiles_m + m_pieces - 1) / m_pieces;
+    double best = -1.0;
+    for (int tn = GS_FEATS; tn >= 64; tn -= 16) {
+        if (tune_n > 0 && tn != tune_n) continue;
+        const int tiles_n = (N + tn - 1) / tn;
+        const long most_n = GS_TERMS_W / (row * tn);
+        if (most_n < 1) continue;
+        const int fewest = (int)((tiles_n + most_n - 1) / most_n);
+        for (int pieces = fewest; pieces < fewest + 4 && pieces <= tiles_n; ++pieces) {
+            const int nt = (tiles_n + pieces - 1) / pieces;
+            for (int ks = 1; ks <= 8; ++ks) {
+                if (tune_split > 0 ? ks != tune_split : (ks > 1 && kb / ks < 2 * GS_CHAIN)) continue;
+                const long blocks = (long)plan->m_tiles * nt * ks, slots = ks == 1 ? n_sm : ks == 2 ? (long)clusters[ks] * ks : (long)(0.9 * clusters[ks]) * ks;
+                if (slots < ks) continue;
+                // a block of k takes the products' time, a launch its ends, a piece of W a launch more and the gaps between;
+                // clusters of 3 and more found fewer places than the occupancy says (512 x 2560 x 4096 in one round of 144 blocks: 95 us;
+                // 120 blocks: 74); terms beyond the L2 are written to memory
+                const double block = fmax(0.73, 0.58 + 0.00133 * tn);
+                const bool spills = row * ((long)plan->m_tiles * GS_TOKENS + (long)nt * tn) > GS_TERMS_L2;
+                const double cost = m_pieces * (pieces * ((double)((blocks + slots - 1) / slots) * ((kb + ks - 1) / ks * block + (ks > 1 ? 8.5 : 2.5)) + 16.0) +
+                                                (double)K * N * (spills ? 2.1e-6 : 1.2e-6)) + (double)K * M * 1.2e-6;
+                if (best < 0.0 || cost < best) best = cost, plan->tile_n = tn, plan->n_tiles = nt, plan->ksplit = ks;
+            }
+        }
+    }
+    if (best < 0.0) return best;
+    plan->bytes = row * ((long)plan->m_tiles * GS_TOKENS + (long)plan->n_tiles * plan->tile_n);
+    return best;
+}
+
+static int gs_run_terms(const float* A, long lda, const float* W, long ldw, void* C, int c_dtype, long ldc, int M, int N, int K, int epilogue,
+                        const GsPlan& plan, unsigned char* scratch, int* status, cudaStream_t stream) {
+    const int kb = (K + GS_BK - 1) / GS_BK, tiles_m = (M + GS_TOKENS - 1) / GS_TOKENS, tiles_n = (N + plan.tile_n - 1) / plan.tile_n;
+    const int per_split = (kb + plan.ksplit - 1) / plan.ksplit;
+    const int ksplit = (kb + per_split - 1) / per_split;
+    unsigned char* w_terms = scratch + (size_t)kb * 3 * 64 * plan.m_tiles * GS_TOKENS;
+    for (int y = 0; y < tiles_m; y += plan.m_tiles) {
+        const int mt = min(plan.m_tiles, tiles_m - y);
+        for (int x = 0; x < tiles_n; x += plan.n_tiles) {
+            const int nt = min(plan.n_tiles, tiles_n - x);
+            const GsOperand a = {A, lda, y * GS_TOKENS, mt * GS_TOKENS, M, scratch}, w = {W, ldw, x * plan.tile_n, nt * plan.tile_n, N, w_terms};
+            const int a_blocks = x == 0 ? mt * (GS_TOKENS / 64) : 0;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(a_blocks + (w.rows + 63) / 64, (kb + 3) / 4);
+            cfg.blockDim = dim3(256);
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = g_bfi_pdl ? 1 : 0;
+            cudaError_t e = cudaLaunchKernelEx(&cfg, split_terms_kernel, a, w, a_blocks, K);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                return bfi_fail("gemm_split: launch failed: %s", cudaGetErrorString(e));
+            }
+            const int rc = gs_launch(gemm_split_kernel<0>, dim3(nt, mt, ksplit), A, lda, W, ldw, C, c_dtype, ldc, M, N, K, plan.tile_n, per_split,
+                                     epilogue, GsTerms{scratch, w_terms, a.rows, w.rows, x, y}, status, stream);
+            if (rc != 0) return rc;
+        }
+    }
+    return 0;
+}
+
+// Bytes of scratch with which bfi_gemm_split_f32 splits both operands ahead of the product; 0: it cannot, or (without `force`)
+// splitting them as it goes takes less time by the estimates.
+extern "C" int bfi_gemm_split_scratch(int M, int N, int K, int force, int tune_n, int tune_split, long* bytes) {
+    BFI_REQUIRE(bytes != nullptr, "gemm_split: no place for the size");
+    *bytes = 0;
+    if (M <= 0 || N <= 0 || K < GS_MIN_K || K % 4 != 0) return 0;
+    GsPlan plan;
+    const double ahead = gs_plan(M, N, K, tune_n, tune_split, &plan);
+    if (ahead < -1.0) return 1;
+    if (ahead < 0.0) return 0;
+    int tile_n, ksplit;
+    if (!force && ahead >= 0.95 * gs_tile(M, N, K, tune_n, tune_split, &tile_n, &ksplit)) return 0;
+    *bytes = plan.bytes;
+    return 0;
+}
+
 // Returns 0 on success, 1 on error, 2 when the product is not taken (nothing launched): rows that are not whole
 // 16-byte pieces, sums shorter than GS_MIN_K, and up to 16 rows, which are bound by reading W and belong to the row
 // kernel of gemm_simt.cu.
 // `tune_n`, `tune_split`: the tile's width and the splits of K, for tests and measurements (0: chosen here).
 extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long ldw, void* C, int c_dtype, long ldc, int M, int N, int K,
-                                  int epilogue, int tune_n, int tune_split, int* status, cudaStream_t stream) {
+                                  int epilogue, int tune_n, int tune_split, void* scratch, long scratch_bytes, int* status,
+                                  cudaStream_t stream) {
     BFI_REQUIRE(dtype_ok(c_dtype), "gemm_split: unknown output dtype code %d", c_dtype);
     BFI_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
     BFI_REQUIRE(lda >= K && ldw >= K, "gemm_split: a row stride is shorter than K=%d", K);
@@ -408,59 +648,24 @@ extern "C" int bfi_gemm_split_f32(const float* A, long lda, const float* W, long
     if (M <= 16 || K < GS_MIN_K || K % 4 != 0 || lda % 4 != 0 || ldw % 4 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return 2;
     const int tiles_m = (M + GS_TOKENS - 1) / GS_TOKENS;
     if (tiles_m > 65535) return 2;
-
-    // the tile's width and the splits of K that take the least time by an estimate: rounds over the SMs x (blocks
-    // of k x 12 products, which take nearly as long for 128 features as for 256, + what surrounds them)
-    const int kb = (K + GS_BK - 1) / GS_BK, n_sm = bfi_sm_count();
-    const int* clusters = gs_clusters<4>();
-    if (clusters == nullptr || gs_clusters<1>() == nullptr || gs_clusters<2>() == nullptr || gs_clusters<3>() == nullptr) return 1;
-    int tile_n = GS_FEATS, ksplit = 1;
-    double best = -1.0;
-    for (int ks = 1; ks <= 8; ++ks) {
-        if (tune_split > 0 ? ks != tune_split : (ks > 1 && kb / ks < 2 * GS_CHAIN)) continue;
-        for (int tn = GS_FEATS; tn >= 64; tn -= 16) {
-            if (tune_n > 0 && tn != tune_n) continue;
-            const long blocks = (long)tiles_m * ((N + tn - 1) / tn) * ks;
-            const long slots = ks == 1 ? n_sm : (long)clusters[ks] * ks;
-            if (slots < ks) continue;
-            const double cost = (double)((blocks + slots - 1) / slots) * ((double)((kb + ks - 1) / ks) * (1.10 + 0.0026 * tn) + (ks > 1 ? 8.5 : 2.5));
-            if (best < 0.0 || cost < best) best = cost, tile_n = tn, ksplit = ks;
-        }
+    if (scratch != nullptr) {
+        GsPlan plan;
+        if (gs_plan(M, N, K, tune_n, tune_split, &plan) < 0.0) return 2;
+        BFI_REQUIRE(scratch_bytes >= plan.bytes && ((uintptr_t)scratch & 15) == 0, "gemm_split: %ld bytes of scratch, %ld needed", scratch_bytes, plan.bytes);
+        return gs_run_terms(A, lda, W, ldw, C, c_dtype, ldc, M, N, K, epilogue, plan, (unsigned char*)scratch, status, stream);
     }
+
+    const int kb = (K + GS_BK - 1) / GS_BK;
+    int tile_n = GS_FEATS, ksplit = 1;
+    const double best = gs_tile(M, N, K, tune_n, tune_split, &tile_n, &ksplit);
+    if (best < -1.0) return 1;
     BFI_REQUIRE(best >= 0.0, "gemm_split: no tile of %d features or no %d splits", tune_n, tune_split);
     const int per_split = (kb + ksplit - 1) / ksplit;
     ksplit = (kb + per_split - 1) / per_split;             // no empty splits
 
     auto kernel = tile_n <= 64 ? gemm_split_kernel<1> : tile_n <= 128 ? gemm_split_kernel<2> : tile_n <= 192 ? gemm_split_kernel<3> : gemm_split_kernel<4>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((N + tile_n - 1) / tile_n, tiles_m, ksplit);
-    cfg.blockDim = dim3(GS_THREADS);
-    cfg.dynamicSmemBytes = GS_SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    int n_attr = 0;
-    if (ksplit > 1) {
-        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-        attr[n_attr].val.clusterDim.x = 1;
-        attr[n_attr].val.clusterDim.y = 1;
-        attr[n_attr].val.clusterDim.z = ksplit;
-        ++n_attr;
-    }
-    if (g_bfi_pdl) {
-        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-        ++n_attr;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    const int vec_ok = (ldc % 4 == 0 && ((uintptr_t)C & 15) == 0) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split, epilogue, vec_ok,
-                                       g_bfi_gate, status);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return bfi_fail("gemm_split: launch failed: %s", cudaGetErrorString(e));
-    }
-    return bfi_check_launch("gemm_split");
+    return gs_launch(kernel, dim3((N + tile_n - 1) / tile_n, tiles_m, ksplit), A, lda, W, ldw, C, c_dtype, ldc, M, N, K, tile_n, per_split,
+                     epilogue, GsTerms{}, status, stream);
 }
 
 BFI_TRACE_EXPORT(gemm_split)

@@ -5,7 +5,7 @@ Nothing here computes anything, and nothing falls back to another implementation
 """
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_long, c_void_p
+from ctypes import byref, c_float, c_int, c_long, c_void_p
 from typing import Optional
 
 import torch
@@ -1092,10 +1092,15 @@ def tc_status(device) -> torch.Tensor:
     return t
 
 
-def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, tile_n: int = 0, splits: int = 0) -> bool:
+SPLIT_AHEAD_MIN_ROWS = 128              # a row of W is split once a tile of 128 tokens: with one tile nothing is split twice
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, tile_n: int = 0, splits: int = 0,
+               ahead: bool | None = None) -> bool:
     """``out = a @ w.T`` for float32 operands on the tensor cores, every operand split exactly into three bfloat16
     terms.  False for products it does not take (up to 16 rows; sums shorter than 512; rows that are not whole 16-byte pieces).
-    ``tile_n``, ``splits``: the tile's width and the splits of K, for tests and measurements (0: the kernel's choice)."""
+    ``tile_n``, ``splits``: the tile's width and the splits of K, ``ahead``: whether the operands are split before the product rather
+    than in it, for tests and measurements (0, None: the kernel's choice)."""
     _need_cuda(a, w, out)
     _rows_2d(a, "A")
     _rows_2d(w, "W")
@@ -1109,9 +1114,20 @@ def gemm_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: in
     cols = n // 2 if epilogue == EPI_SWIGLU else n
     if out.shape != (m, cols):
         raise KernelError(f"matrix product: output must be [{m}, {cols}], got {tuple(out.shape)}")
+    scratch = None
+    if ahead or (ahead is None and m > SPLIT_AHEAD_MIN_ROWS):
+        need = c_long(0)
+        library("core").call("bfi_gemm_split_scratch", c_int(m), c_int(n), c_int(k), c_int(1 if ahead else 0), c_int(tile_n), c_int(splits),
+                             byref(need))
+        if need.value:
+            try:
+                scratch = torch.empty(need.value, dtype=torch.uint8, device=a.device)
+            except torch.OutOfMemoryError:
+                pass                                       # the product splits its operands as it goes
     return library("core").call_optional(
         "bfi_gemm_split_f32", _ptr(a), c_long(a.stride(0)), _ptr(w), c_long(w.stride(0)), _ptr(out), c_int(dtype_code(out.dtype)),
-        c_long(out.stride(0)), c_int(m), c_int(n), c_int(k), c_int(epilogue), c_int(tile_n), c_int(splits), _ptr(tc_status(a.device)),
+        c_long(out.stride(0)), c_int(m), c_int(n), c_int(k), c_int(epilogue), c_int(tile_n), c_int(splits),
+        _ptr(scratch), c_long(scratch.numel() if scratch is not None else 0), _ptr(tc_status(a.device)),
         _stream())
 
 

@@ -81,3 +81,30 @@ def test_what_it_leaves_to_the_other_kernels(m, n, k):
     assert not ops.gemm_split(a, w, out)
     linear(a, w, out)
     assert err(out, a.double() @ w.double().T) < 1e-6
+
+
+@pytest.mark.parametrize("m,n,k,tile_n,splits", [
+    (1, 64, 512, 64, 1), (129, 257, 516, 256, 1), (300, 1000, 1000, 208, 2), (513, 2000, 2728, 0, 0), (640, 9000, 2560, 0, 0),
+    (5000, 130, 4100, 0, 0)])               # the last two: several pieces of W, of A
+def test_operands_split_ahead_give_the_same_sums(m, n, k, tile_n, splits):
+    from builderforce_inference_b200.kernels import ops
+    a, w = operands(max(m, 17), n, k, 8, wide=True)
+    ref = a.double() @ w.double().T
+    out = torch.full((a.shape[0], n + 4), 7.0, device=DEV)
+    assert ops.gemm_split(a, w, out[:, :n], ops.EPI_STORE, tile_n, splits, ahead=True)
+    assert int(ops.tc_status(DEV)[0].item()) == 0
+    assert torch.all(out[:, n:] == 7.0)
+    assert err(out[:, :n], ref) < 3e-7
+    if tile_n:                              # the same terms, products, chains and order
+        plain = torch.empty(a.shape[0], n, device=DEV)
+        assert ops.gemm_split(a, w, plain, ops.EPI_STORE, tile_n, splits, ahead=False)
+        assert torch.equal(out[:, :n], plain)
+    old = torch.randn(a.shape[0], n, device=DEV)
+    acc = old.clone()
+    assert ops.gemm_split(a, w, acc, ops.EPI_ACCUMULATE, tile_n, splits, ahead=True) and err(acc, ref + old.double()) < 3e-7
+    if n % 2 == 0:
+        gated = torch.empty(a.shape[0], n // 2, device=DEV)
+        assert ops.gemm_split(a, w, gated, ops.EPI_SWIGLU, tile_n, splits, ahead=True)
+        half = torch.empty_like(gated)
+        assert ops.gemm_split(a, w, half, ops.EPI_SWIGLU, tile_n, splits, ahead=False)
+        assert err(gated, half.double()) < 6e-7
