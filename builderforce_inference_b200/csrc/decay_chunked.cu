@@ -24,6 +24,9 @@
 //     32 heads, one prompt of 2,048 tokens, a decay per head: 757 -> 119 us; per row: 770 -> 233 us
 //     16 heads, prompts of 1,500, 1,043, 587 and 130 tokens, a decay per row: 548 -> 210 us
 //     16 heads, 8 prompts of 33 to 500 tokens, a decay per head: 360 -> 74 us
+// and, for constant decays, lightning_chunked.cu (which walks the chunks of a sequence) -> these kernels:
+//     32 heads, one prompt of 2,048 tokens: 203 -> 140 us; three of 301 to 2,048: 296 -> 268 (122 MB of scratch: the L2 no longer holds it)
+//     16 heads, one prompt of 2,048 tokens: 151 ->  70 us, of 4,096: 303 -> 143
 // Distance from a 64-bit walk, relative to the 2-norm (2,048 tokens; a float32 walk in order in brackets): outputs 1.3e-7
 // (1.8e-7), state 0.9e-7 (1.5e-7); a decay per row: 1.9e-7 (2.1e-7), 1.7e-7 (1.8e-7).
 #include "chunk_tiles.cuh"
@@ -31,6 +34,7 @@
 #define DC_LEN 64            // tokens per chunk
 #define DC_STEP 1            // REC_DECAY_STEP and REC_DECAY_SIGMOID of recurrence.cu
 #define DC_SIGMOID 2
+#define DC_FIXED 3           // a constant per head (lightning.cu), q, k and v activated as they are read
 #define DC_LDP (DC_LEN + 8)
 #define DC_SMALLEST 8.2718061255302767e-25f      // 2^-80
 // Warps of a block: eight, two blocks on an SM; sixteen where three terms of queries and keys leave room for one block
@@ -41,12 +45,20 @@ struct DcArgs {
     int q_off, k_off, v_off, r_off;
     int H, D, V, heads_per_group, v_blocks;
     float q_scale, inv_tau;
-    const float *bias, *rate, *skip;
+    const float *bias, *rate, *skip;                     // DC_FIXED: `rate` holds the decays
+    int silu;
     const int *cu_seqlens, *seq_slot;
 };
 
 __device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
 __device__ __forceinline__ float dc_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
+// as lightning_chunked.cu activates: rounded to bfloat16
+__device__ __forceinline__ uint32_t dc_silu(uint32_t x) {
+    const float a = bf16_lo(x), b = bf16_hi(x);
+    const __nv_bfloat162 y = __floats2bfloat162_rn(__fdividef(a, 1.0f + __expf(-a)), __fdividef(b, 1.0f + __expf(-b)));
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+__device__ __forceinline__ uint4 dc_silu(uint4 x) { return make_uint4(dc_silu(x.x), dc_silu(x.y), dc_silu(x.z), dc_silu(x.w)); }
 // any of eight bfloat16 values infinite or NaN
 __device__ __forceinline__ bool dc_not_finite(uint4 x) {
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
@@ -95,6 +107,10 @@ __device__ __noinline__ void plain_chunk(float* sm, const bf16* __restrict__ qk,
     const int grp = h / a.heads_per_group;
     const float skip = a.skip ? a.skip[h] : 0.0f;
     float prod = 1.0f;
+    auto value = [&](bf16 x) {
+        if (MODE == DC_FIXED && a.silu) return bf16_lo(dc_silu((uint32_t)__bfloat16_as_ushort(x)));
+        return to_f32(x);
+    };
     __syncthreads();
     for (int i = tid; i < D * VB; i += THREADS) S[i] = OUT ? start[(size_t)(i / VB) * a.V + i % VB] : 0.0f;
     for (int t = 0; t < n; ++t) {
@@ -103,16 +119,17 @@ __device__ __noinline__ void plain_chunk(float* sm, const bf16* __restrict__ qk,
         if (tid == 0) *step = MODE == DC_STEP ? dc_softplus(to_f32(raw[tok * a.r_stride + a.r_off + h]) + a.bias[h]) : 1.0f;
         __syncthreads();
         if (tid < D) {
-            const float w = MODE == DC_STEP ? expf(-a.rate[h] * *step)
-                                            : expf(dc_log_sigmoid(to_f32(raw[tok * a.r_stride + a.r_off + (size_t)h * D + tid]) +
+            const float w = MODE == DC_FIXED ? a.rate[h]
+                          : MODE == DC_STEP  ? expf(-a.rate[h] * *step)
+                                             : expf(dc_log_sigmoid(to_f32(raw[tok * a.r_stride + a.r_off + (size_t)h * D + tid]) +
                                                                   a.bias[(size_t)h * D + tid]) * a.inv_tau);
-            qs[tid] = OUT ? to_f32(qk[tok * a.qk_stride + a.q_off + (size_t)grp * D + tid]) * a.q_scale : 0.0f;
-            ks[tid] = to_f32(qk[tok * a.qk_stride + a.k_off + (size_t)grp * D + tid]);
+            qs[tid] = OUT ? value(qk[tok * a.qk_stride + a.q_off + (size_t)grp * D + tid]) * a.q_scale : 0.0f;
+            ks[tid] = value(qk[tok * a.qk_stride + a.k_off + (size_t)grp * D + tid]);
             as[tid] = w;
             prod *= w;
         }
         __syncthreads();
-        const float vv = to_f32(vsrc[tok * a.v_stride + a.v_off + (size_t)h * a.V + v0 + c]);
+        const float vv = value(vsrc[tok * a.v_stride + a.v_off + (size_t)h * a.V + v0 + c]);
         float acc = 0.0f;
         if (g < ng) {
             for (int d = g; d < D; d += ng) {
@@ -208,13 +225,25 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
     for (int u = 0; u < NP; ++u) bad |= dc_not_finite(xq[u]) || dc_not_finite(xk[u]);
 #pragma unroll
     for (int u = 0; u < NV; ++u) bad |= dc_not_finite(xv[u]);
-    if (MODE == DC_STEP) {
+    if (MODE == DC_FIXED && a.silu) {
+#pragma unroll
+        for (int u = 0; u < NP; ++u) xq[u] = dc_silu(xq[u]), xk[u] = dc_silu(xk[u]);
+#pragma unroll
+        for (int u = 0; u < NV; ++u) xv[u] = dc_silu(xv[u]);
+    }
+    if (MODE != DC_SIGMOID) {
         if (warp == 0) {                                 // log decays summed over the chunk: two tokens a lane
             float c2[2];
             double l2[2];
+            const double each = MODE == DC_FIXED ? log((double)a.rate[h]) : 0.0;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int t = 2 * lane + i;
+                if (MODE == DC_FIXED) {
+                    c2[i] = t < n ? 1.0f : 0.0f;
+                    l2[i] = t < n ? each : 0.0;
+                    continue;
+                }
                 c2[i] = t < n ? dc_softplus(to_f32(raw[(size_t)(t0 + t) * a.r_stride + a.r_off + h]) + a.bias[h]) : 0.0f;
                 l2[i] = t < n ? (double)(-a.rate[h] * c2[i]) : 0.0;
             }
@@ -225,7 +254,7 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
                 if (lane >= o) run += up;
             }
             const double all = __shfl_sync(0xffffffffu, run, 31);
-            bad |= !(all > -1e30);                       // an infinite step leaves no difference to take
+            bad |= !(all > -1e30);                       // an infinite step (a decay of zero, or below it) leaves no difference to take
             cum[2 * lane] = run - l2[1], cum[2 * lane + 1] = run;
             cs[2 * lane] = c2[0], cs[2 * lane + 1] = c2[1];
             if (OUT) {
@@ -322,9 +351,9 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
 
     if (!OUT) {
         if (v0 == 0)
-            for (int d = tid; d < D; d += THREADS) my_decay[d] = MODE == DC_STEP ? tot[0] : tot[d] * tot[D + d];
+            for (int d = tid; d < D; d += THREADS) my_decay[d] = MODE != DC_SIGMOID ? tot[0] : tot[d] * tot[D + d];
         if (!has_columns) return;
-        constexpr int BT = MODE == DC_STEP ? 3 : 1;      // terms of (c v); v itself is one
+        constexpr int BT = MODE != DC_SIGMOID ? 3 : 1;      // terms of (c v); v itself is one
         uint32_t b[4][BT][4];
 #pragma unroll
         for (int kj = 0; kj < 4; ++kj) {
@@ -333,7 +362,7 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int j = kj * 16 + t2 + (i & 1) * 8;
-                if (MODE == DC_STEP)
+                if (MODE != DC_SIGMOID)
                     split_pair(bf16_lo(raw4[i]) * ws[j], bf16_hi(raw4[i]) * ws[j + 1], b[kj][0][i], b[kj][BT > 1 ? 1 : 0][i], b[kj][BT > 2 ? 2 : 0][i]);
                 else
                     b[kj][0][i] = raw4[i];
@@ -418,7 +447,7 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     float f = a.q_scale;
-                    if (MODE == DC_STEP) f *= cs[j + i] * expf((float)(cum[t] - cum[min(j + i, t)]));
+                    if (MODE != DC_SIGMOID) f *= cs[j + i] * expf((float)(cum[t] - cum[min(j + i, t)]));
                     x[i] = j + i <= t ? ((hi[0][nb][2 * r + i] + hi[1][nb][2 * r + i]) + lo[nb][2 * r + i]) * f : 0.0f;
                 }
                 uint32_t th, tm, tl;
@@ -501,7 +530,7 @@ decay_chunk_kernel(const bf16* __restrict__ qk, const bf16* __restrict__ vsrc, c
         for (int r = 0; r < 2; ++r) {
             const int t = ti * 16 + g + r * 8;
             if (t >= n) continue;
-            const float f = MODE == DC_STEP ? ws[t] : a.q_scale;
+            const float f = MODE != DC_SIGMOID ? ws[t] : a.q_scale;
 #pragma unroll
             for (int nb = 0; nb < 2; ++nb) {
                 const uint32_t v2 = *reinterpret_cast<const uint32_t*>(Vs + t * L.ldv + vt * 16 + nb * 8 + t2);
@@ -587,7 +616,7 @@ extern "C" int bfi_decay_chunks_bf16(const void* qk, long qk_stride, int q_off, 
     if (((uintptr_t)qk & 15) || ((uintptr_t)vsrc & 15) || qk_stride % 8 || v_stride % 8 || q_off % 8 || k_off % 8 || v_off % 8) return 2;
     if (((uintptr_t)out & 7) || out_stride % 2 || ((uintptr_t)state & 15) || ((uintptr_t)chunk_state & 15)) return 2;
     if (mode == DC_SIGMOID && (((uintptr_t)raw & 15) || r_stride % 8 || r_off % 8 || ((uintptr_t)bias & 15))) return 2;
-    DcArgs a;
+    DcArgs a = {};
     a.qk_stride = qk_stride, a.v_stride = v_stride, a.r_stride = r_stride, a.out_stride = out_stride;
     a.q_off = q_off, a.k_off = k_off, a.v_off = v_off, a.r_off = r_off;
     a.H = H, a.D = D, a.V = V, a.heads_per_group = heads_per_group, a.v_blocks = (V + 127) / 128;
@@ -603,6 +632,29 @@ extern "C" int bfi_decay_chunks_bf16(const void* qk, long qk_stride, int q_off, 
     if (D <= 64) BFI_DC(DC_SIGMOID, 64);
     BFI_DC(DC_SIGMOID, 128);
 #undef BFI_DC
+}
+
+// The arguments of bfi_lightning_scan for bfloat16 projections without a rotation, with scratch as above.
+extern "C" int bfi_fixed_decay_chunks_bf16(const void* proj, long stride, int q_off, int k_off, int v_off, float* out, long out_stride,
+                                           float* state, const float* decay, const int* cu_seqlens, const int* seq_slot, int n_seqs, int H,
+                                           int D, int V, int silu, int max_chunks, float* chunk_state, float* chunk_decay, cudaStream_t stream) {
+    BFI_REQUIRE(H > 0 && D > 0 && V > 0, "decay_chunks: bad sizes heads=%d dim=%d vdim=%d", H, D, V);
+    BFI_REQUIRE(decay != nullptr, "decay_chunks: the decays are missing");
+    BFI_REQUIRE(out_stride >= (long)H * V, "decay_chunks: output stride shorter than the heads");
+    BFI_REQUIRE(max_chunks > 0 && chunk_state != nullptr && chunk_decay != nullptr, "decay_chunks: the chunks' count and scratch are missing");
+    if (n_seqs <= 0) return 0;
+    if (D % 16 != 0 || D > 128 || V % 16 != 0 || n_seqs > 65535 || max_chunks > 65535 || H > 65535) return 2;
+    if (((uintptr_t)proj & 15) || stride % 8 || q_off % 8 || k_off % 8 || v_off % 8) return 2;
+    if (((uintptr_t)out & 7) || out_stride % 2 || ((uintptr_t)state & 15) || ((uintptr_t)chunk_state & 15)) return 2;
+    DcArgs a = {};
+    a.qk_stride = a.v_stride = stride, a.out_stride = out_stride;
+    a.q_off = q_off, a.k_off = k_off, a.v_off = v_off;
+    a.H = H, a.D = D, a.V = V, a.heads_per_group = 1, a.v_blocks = (V + 127) / 128;
+    a.q_scale = 1.0f, a.rate = decay, a.silu = silu;
+    a.cu_seqlens = cu_seqlens, a.seq_slot = seq_slot;
+    const bf16* p = (const bf16*)proj;
+    if (D <= 64) return launch_decay_chunks<DC_FIXED, 64>(p, p, nullptr, out, state, chunk_state, chunk_decay, a, n_seqs, max_chunks, stream);
+    return launch_decay_chunks<DC_FIXED, 128>(p, p, nullptr, out, state, chunk_state, chunk_decay, a, n_seqs, max_chunks, stream);
 }
 
 BFI_TRACE_EXPORT(decay_chunked)

@@ -352,6 +352,51 @@ def attention_prefill_tcgen05_wait_probe(ctx, qkv: torch.Tensor, out: torch.Tens
 LIGHTNING_CHUNK_MIN_TOKENS = 8     # shorter runs of new tokens: the token-by-token kernel
 
 
+FIXED_CHUNKS_MAX_BYTES = 256 << 20     # scratch for the chunks' states: more tokens than that are walked
+
+
+def fixed_decay_chunks_pay(longest: int, n_chunks: int, n_seqs: int, n_heads: int, dim: int, vdim: int) -> bool:
+    """Whether chunks side by side take less time than a walk over each sequence's, by an estimate in us.  ``longest``: chunks of the
+    longest sequence.  A walk takes 9.2, 6.3 or 4.7 us a chunk for 64, 32 or 16 columns a block (0.7 of it for heads of up to 64) over
+    the longest sequence or over all rounds; side by side it is three launches and, beyond 256 chunks of heads, the work and the
+    scratch of each.  Fewer than 5 chunks never gained (4 sequences of 64 tokens, 32 heads: 27 / 41).  Measured, walk / side by side: 32 heads of 128 x 128, a prompt of 2,048 tokens 203 / 140, of 300 34 / 35, three of
+    301 to 2,048 296 / 268, 16 of 200 291 / 353; 16 heads, one of 2,048 151 / 70, one of 4,096 303 / 143; 16 heads of 64 x 64, one
+    of 2,048 105 / 41, 16 of 500 106 / 134; 8 heads of 128 x 64, one of 500 40 / 27, of 200 21 / 27."""
+    if longest < 5 or n_chunks * n_heads * dim * vdim * 4 > FIXED_CHUNKS_MAX_BYTES:
+        return False
+    per_block, per_chunk, best = 16, 4.7, None
+    for cols, us in ((64, 9.2), (32, 6.3), (16, 4.7)):
+        if vdim % cols == 0:
+            cost = -(-n_seqs * n_heads * (vdim // cols) // 148) * us
+            if best is None or cost < best:
+                best, per_block, per_chunk = cost, cols, us
+    walk = per_chunk * (0.7 if dim <= 64 else 1.0) * max(longest, -(-(n_chunks - n_seqs) * n_heads * (vdim // per_block) // 148))
+    k = dim * vdim / 1024
+    side = 14 + 1.2 * k + max(0, n_chunks * n_heads - 256) * (0.03 + 0.0062 * k)
+    return 1.1 * side < walk
+
+
+def fixed_decay_chunks_bf16(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor,
+                            decay: torch.Tensor, cu_seqlens: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int, n_heads: int, dim: int,
+                            vdim: int, act: int, max_chunks: int, chunk_state: torch.Tensor, chunk_decay: torch.Tensor) -> bool:
+    """``lightning_chunks_bf16`` without a rotation or scale, the chunks of a sequence side by side: ``chunk_state`` and
+    ``chunk_decay`` are ``ops.decay_scan``'s scratch for every chunk of 64 tokens.  False for sizes it does not take."""
+    if proj.dtype != torch.bfloat16 or out.dtype != torch.float32 or state.dtype != torch.float32:
+        return False
+    _rows_2d(proj, "projections")
+    _rows_2d(out, "recurrence output")
+    if not state.is_contiguous() or tuple(state.shape[1:]) != (n_heads, dim, vdim) or out.shape[1] != n_heads * vdim:
+        raise KernelError("fixed_decay_chunks: state [slots, heads, dim, vdim] and output [tokens, heads * vdim] expected")
+    n_chunks = proj.shape[0] // 64 + n_seqs
+    for t, per in ((chunk_state, n_heads * dim * vdim), (chunk_decay, n_heads * dim)):
+        if t.dtype != torch.float32 or not t.is_contiguous() or t.numel() < n_chunks * per or not t.is_cuda:
+            raise KernelError(f"fixed_decay_chunks: float32 scratch for {n_chunks} chunks expected")
+    return library("fast").call_optional(
+        "bfi_fixed_decay_chunks_bf16", _ptr(proj), c_long(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), _ptr(out),
+        c_long(out.stride(0)), _ptr(state), _ptr(decay), _ptr(cu_seqlens), _ptr(seq_slot), c_int(n_seqs), c_int(n_heads), c_int(dim),
+        c_int(vdim), c_int(1 if act == LIGHT_ACT_SILU else 0), c_int(max_chunks), _ptr(chunk_state), _ptr(chunk_decay), _stream())
+
+
 def lightning_chunks_bf16(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor,
                           decay: torch.Tensor, cu_seqlens: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int,
                           n_heads: int, dim: int, vdim: int, act: int = LIGHT_ACT_SILU, rope_table=None, rot_dim: int = 0,

@@ -111,3 +111,57 @@ def test_gated_norm_of_rows_in_whole_groups(dt, width):
     ops.gated_rmsnorm(x, gate, w, 1e-5, out)
     ref = x.to(F64) * torch.rsqrt(x.to(F64).square().mean(1, keepdim=True) + 1e-5) * w.to(F64) * torch.sigmoid(gate.to(F64))
     assert err(out, ref) < (5e-7 if dt == torch.float32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("lens,H,D,V,decay", [
+    ([1], 2, 16, 16, [0.9, 0.5]), ([64, 65, 200], 2, 64, 48, [0.999, 0.6]), ([63, 130, 7], 3, 48, 144, [1.0, 0.93, 0.05]),
+    ([700, 9], 2, 128, 128, [0.97, 0.0])])          # a decay of zero: token by token
+@pytest.mark.parametrize("act", [0, 1])
+def test_constant_decays_side_by_side(lens, H, D, V, decay, act):
+    from builderforce_inference_b200.kernels import fast_ops
+    g = torch.Generator(device=DEV).manual_seed(sum(lens) + D)
+    n, at = sum(lens), 0
+    proj = torch.randn(n, 2 * H * D + H * V, generator=g, device=DEV).bfloat16()
+    dec = torch.tensor(decay, device=DEV)
+    first = 0.3 * torch.randn(len(lens) + 1, H, D, V, generator=g, device=DEV)
+    x = proj.to(F64)
+    if act:
+        x = torch.nn.functional.silu(x).bfloat16().to(F64)
+    ref, ends = [], []
+    for i, m in enumerate(lens):
+        S = first[i + 1].to(F64)
+        for t in range(at, at + m):
+            q, k, v = x[t, :H * D].view(H, D), x[t, H * D:2 * H * D].view(H, D), x[t, 2 * H * D:].view(H, V)
+            S = dec.to(F64)[:, None, None] * S + k[:, :, None] * v[:, None]
+            ref.append((q[:, None] @ S).reshape(-1))
+        at += m
+        ends.append(S)
+    ref, ends = torch.stack(ref), torch.stack(ends)
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    slots = torch.arange(1, len(lens) + 1, dtype=torch.int32, device=DEV)
+    chunks = n // 64 + len(lens)
+    rel = lambda a, b: float((a.to(F64) - b).norm() / b.norm())  # noqa: E731
+
+    def run(proj, side_by_side):
+        out, state = torch.full((n, H * V), float("nan"), device=DEV), first.clone()
+        args = (proj, 0, H * D, 2 * H * D, out, state, dec, cu, slots, len(lens), H, D, V)
+        if side_by_side:
+            assert fast_ops.fixed_decay_chunks_bf16(*args, act, (max(lens) + 63) // 64, torch.full((chunks, H * D * V), float("nan"), device=DEV),
+                                                    torch.full((chunks, H * D), float("nan"), device=DEV))
+        else:
+            assert fast_ops.lightning_chunks_bf16(*args, act=act)
+        assert torch.equal(state[0], first[0])
+        return out, state
+
+    out, state = run(proj, True)
+    walk, walked = run(proj, False)
+    # silu is made with the fast exponential in both: a value in some hundreds rounds to the neighbouring bfloat16
+    limit = 1e-4 if act else 5e-7
+    assert rel(out, ref) < limit and rel(state[1:], ends) < limit
+    assert rel(out, ref) <= rel(walk, ref) * 1.01 and rel(state[1:], ends) <= rel(walked[1:], ends) * 1.01
+    # a token that is not finite reaches nothing before it and no other sequence
+    proj[-2 if lens[-1] > 1 else -1, H * D] = float("inf")
+    bad, _ = run(proj, True)
+    cut = n - (2 if lens[-1] > 1 else 1)
+    assert torch.isfinite(bad[:cut]).all() and not torch.isfinite(bad[-1, :V]).all()
+    assert rel(bad[:cut], ref[:cut]) < limit if cut else True
